@@ -27,8 +27,6 @@
 namespace {
 
 constexpr int kGraphSteps = 16;  // steps per replay of the long graph
-// launches per step: dt, four stages each followed by its ghost pass, finish
-constexpr int kLaunchesPerStep = 10;
 
 __global__ void batch_dt_kernel(BatchInst *tab, long long *left, int *status, int n, int D) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -128,9 +126,16 @@ struct smaug_batch {
   std::vector<BatchInst> h_tab;
   std::vector<Slot> slots;
   WorkItem *d_work = nullptr;
-  WorkItem *d_gwork = nullptr;  // ghost chunks (256 ghost cells of one simulation each)
-  size_t gwork_cap = 0;
-  int ngwork = 0, ggrid = 0;
+  WorkItem *d_awork = nullptr;  // advance chunks
+  size_t awork_cap = 0;
+  // 3-D: the plan of a stage over the current simulations, its slab list on
+  // the device (its items are d_work) and the workspace
+  Plan3 plan3;
+  Slab3 *d_slabs = nullptr;
+  size_t slabs_cap = 0;
+  char *work3 = nullptr;
+  size_t work3_bytes = 0;
+  int nawork = 0;
   size_t work_cap = 0;
   int nwork = 0, grid = 0, variant = 0, sms = 148;
   bool dirty = true;
@@ -159,8 +164,10 @@ struct smaug_batch {
   int last_snap = -1;  // ring entry of the last snapshot waited for (asynchronous reads follow it)
   // pinned staging of the work lists and the table (two sets, used in turn)
   BatchInst *st_tab[2] = {};
-  WorkItem *st_work[2] = {}, *st_gwork[2] = {};
-  size_t st_work_cap[2] = {}, st_gwork_cap[2] = {};
+  WorkItem *st_work[2] = {}, *st_awork[2] = {};
+  Slab3 *st_slabs[2] = {};
+  size_t st_slabs_cap[2] = {};
+  size_t st_work_cap[2] = {}, st_awork_cap[2] = {};
   cudaEvent_t st_ev[2] = {};
   int st_cur = 0;
 };
@@ -220,16 +227,26 @@ void set_tiles(const smaug_batch *b, BatchInst &I) {
   for (int d = 0; d < 3; ++d) I.tiles[d] = d < b->D ? (I.geo.n[d] - 4 + t[d] - 1) / t[d] : 1;
 }
 
-// Rebuild the work list and the persistent grid for the current simulations
-// and tile shape.
-// Grow pinned staging buffer k of `what` (its copies from two rebuilds ago
-// are done: the caller waited for st_ev[k]).
-int stage_grow(smaug_batch *b, WorkItem **buf, size_t *cap, size_t need) {
+// Grow a pinned staging buffer (its copies from two rebuilds ago are done: the
+// caller waited for its event).
+template <typename E>
+int stage_grow(smaug_batch *b, E **buf, size_t *cap, size_t need) {
   if (need <= *cap) return SMAUG_OK;
   if (*buf) cudaFreeHost(*buf);
   *buf = nullptr;
   *cap = std::max(need, (size_t)1024) * 2;
-  BK(cudaMallocHost((void **)buf, sizeof(WorkItem) * *cap));
+  BK(cudaMallocHost((void **)buf, sizeof(E) * *cap));
+  return SMAUG_OK;
+}
+
+// Grow a device list (the caller waited for the steps that read it).
+template <typename E>
+int list_grow(smaug_batch *b, E **list, size_t *cap, size_t need) {
+  if (need <= *cap) return SMAUG_OK;
+  cudaFree(*list);
+  *list = nullptr;
+  *cap = std::max(need, (size_t)1024) * 2;
+  BK(cudaMalloc(list, sizeof(E) * *cap));
   return SMAUG_OK;
 }
 
@@ -239,54 +256,78 @@ int stage_grow(smaug_batch *b, WorkItem **buf, size_t *cap, size_t need) {
 // steps already queued, except when a device list must grow.
 int rebuild(smaug_batch *b) {
   std::vector<WorkItem> w, gw;
+  std::vector<std::pair<int, Geo>> sims;
   for (int i = 0; i < b->max_inst; ++i) {
     if (!b->slots[i].used) continue;
     set_tiles(b, b->h_tab[i]);
     const int *tl = b->h_tab[i].tiles;
-    for (int z = 0; z < tl[2]; ++z)
+    if (b->D == 3)
+      sims.push_back({i, b->h_tab[i].geo});
+    else
       for (int y = 0; y < tl[1]; ++y)
-        for (int x = 0; x < tl[0]; ++x) w.push_back({i, x, y, z});
-    const long long ng = ghost_cells(b->h_tab[i].geo, b->D);
-    for (long long t = 0; t < (ng + 255) / 256; ++t) gw.push_back({i, (int)t, 0, 0});
+        for (int x = 0; x < tl[0]; ++x) w.push_back({i, x, y, 0});
+    const int na = advance_items(b->h_tab[i].geo, b->D);
+    for (int t = 0; t < na; ++t) gw.push_back({i, t, 0, 0});
   }
-  if (gw.size() > b->gwork_cap || w.size() > b->work_cap) {  // queued steps read the device lists
+  if (b->D == 3) {
+    int t[3];
+    batch_tile_shape(3, b->variant, t);
+    b->plan3.build(sims, t, b->mixed);
+    w.swap(b->plan3.items);
+  }
+  const size_t nslab = b->plan3.slabs.size();
+  int rc = SMAUG_OK;
+  if (gw.size() > b->awork_cap || w.size() > b->work_cap || nslab > b->slabs_cap ||
+      b->plan3.bytes > b->work3_bytes) {  // queued steps read the device lists and use the workspace
     BK(cudaStreamSynchronize(b->stream));
-    if (gw.size() > b->gwork_cap) {
-      if (b->d_gwork) cudaFree(b->d_gwork);
-      b->gwork_cap = std::max(gw.size(), (size_t)1024) * 2;
-      BK(cudaMalloc(&b->d_gwork, sizeof(WorkItem) * b->gwork_cap));
-    }
-    if (w.size() > b->work_cap) {
-      if (b->d_work) cudaFree(b->d_work);
-      b->work_cap = std::max(w.size(), (size_t)1024) * 2;
-      BK(cudaMalloc(&b->d_work, sizeof(WorkItem) * b->work_cap));
+    if ((rc = list_grow(b, &b->d_awork, &b->awork_cap, gw.size())) != SMAUG_OK) return rc;
+    if ((rc = list_grow(b, &b->d_work, &b->work_cap, w.size())) != SMAUG_OK) return rc;
+    if ((rc = list_grow(b, &b->d_slabs, &b->slabs_cap, nslab)) != SMAUG_OK) return rc;
+    if (b->plan3.bytes > b->work3_bytes) {
+      cudaFree(b->work3);
+      b->work3 = nullptr;
+      b->work3_bytes = 0;
+      BK(cudaMalloc(&b->work3, b->plan3.bytes));
+      b->work3_bytes = b->plan3.bytes;
     }
   }
+  b->plan3.place(b->work3);
   const int k = b->st_cur;
   b->st_cur ^= 1;
   BK(cudaEventSynchronize(b->st_ev[k]));  // the copies out of set k, two rebuilds ago
-  int rc = stage_grow(b, &b->st_gwork[k], &b->st_gwork_cap[k], gw.size());
-  if (rc != SMAUG_OK) return rc;
-  rc = stage_grow(b, &b->st_work[k], &b->st_work_cap[k], w.size());
-  if (rc != SMAUG_OK) return rc;
+  if ((rc = stage_grow(b, &b->st_awork[k], &b->st_awork_cap[k], gw.size())) != SMAUG_OK) return rc;
+  if ((rc = stage_grow(b, &b->st_work[k], &b->st_work_cap[k], w.size())) != SMAUG_OK) return rc;
+  if ((rc = stage_grow(b, &b->st_slabs[k], &b->st_slabs_cap[k], nslab)) != SMAUG_OK) return rc;
   std::memcpy(b->st_tab[k], b->h_tab.data(), sizeof(BatchInst) * b->max_inst);
-  if (!gw.empty()) std::memcpy(b->st_gwork[k], gw.data(), sizeof(WorkItem) * gw.size());
-  if (!w.empty()) std::memcpy(b->st_work[k], w.data(), sizeof(WorkItem) * w.size());
-  if (!gw.empty())
-    BK(cudaMemcpyAsync(b->d_gwork, b->st_gwork[k], sizeof(WorkItem) * gw.size(), cudaMemcpyHostToDevice, b->stream));
   BK(cudaMemcpyAsync(b->d_tab, b->st_tab[k], sizeof(BatchInst) * b->max_inst, cudaMemcpyHostToDevice, b->stream));
-  if (!w.empty())
-    BK(cudaMemcpyAsync(b->d_work, b->st_work[k], sizeof(WorkItem) * w.size(), cudaMemcpyHostToDevice, b->stream));
+  auto put = [&](auto *dev, auto *staging, const auto *src, size_t n) {
+    if (n == 0) return cudaSuccess;
+    std::memcpy(staging, src, sizeof(*src) * n);
+    return cudaMemcpyAsync(dev, staging, sizeof(*src) * n, cudaMemcpyHostToDevice, b->stream);
+  };
+  BK(put(b->d_awork, b->st_awork[k], gw.data(), gw.size()));
+  BK(put(b->d_work, b->st_work[k], w.data(), w.size()));
+  BK(put(b->d_slabs, b->st_slabs[k], b->plan3.slabs.data(), nslab));
   BK(cudaEventRecord(b->st_ev[k], b->stream));
-  b->ngwork = (int)gw.size();
-  b->ggrid = std::min(b->ngwork, 148 * 8);
+  b->nawork = (int)gw.size();
   b->nwork = (int)w.size();
   const int occ = std::max(1, smaug_batchk::batch_stage_occupancy(b->D, b->mixed, b->variant));
-  b->grid = std::min(b->nwork, occ * b->sms);
+  b->grid = b->D == 2 ? std::min(b->nwork, occ * b->sms) : occ * b->sms;
   drop_graphs(b);
   b->dirty = false;
   return SMAUG_OK;
 }
+
+// RK stage k of the whole batch on stream s.
+void launch_rk_stage(smaug_batch *b, int k, cudaStream_t s) {
+  if (b->D == 2)
+    smaug_batchk::launch_batch_stage2(b->mixed, b->variant, b->d_tab, b->d_work, b->nwork, k, b->grid, s);
+  else
+    smaug_batchk::launch_pass3(b->mixed, b->variant, b->d_tab, b->d_slabs, b->d_work, b->plan3, k, b->grid, s);
+}
+int launches_per_rk_stage(const smaug_batch *b) { return b->D == 2 ? 1 : 3 * (int)b->plan3.groups.size(); }
+// A step: dt, four stages each followed by its advance pass, finish.
+int launches_per_step(const smaug_batch *b) { return 6 + 4 * launches_per_rk_stage(b); }
 
 // The step stream waits for the admissions queued on the upload stream.
 int join_uploads(smaug_batch *b) {
@@ -347,9 +388,9 @@ void enqueue_step(smaug_batch *b, cudaStream_t s, bool timed = false) {
         b->ev_used += 2;
       }
     }
-    smaug_batchk::launch_batch_stage(b->D, b->mixed, b->variant, b->d_tab, b->d_work, b->nwork, k, b->grid, s);
+    launch_rk_stage(b, k, s);
+    smaug_batchk::launch_batch_advance(b->D, b->mixed, b->d_tab, b->d_awork, b->nawork, k, b->sms, s);
     if (e1) cudaEventRecord(e1, s);
-    smaug_batchk::launch_batch_ghost(b->D, b->mixed, b->d_tab, b->d_gwork, b->ngwork, k, b->ggrid, s);
   }
   batch_finish_kernel<<<nb, 128, 0, s>>>(b->d_tab, b->d_status, b->max_inst);
 }
@@ -437,7 +478,9 @@ int smaug_batch_destroy(smaug_batch *b) {
   cudaFree(b->d_left);
   cudaFree(b->d_status);
   cudaFree(b->d_work);
-  cudaFree(b->d_gwork);
+  cudaFree(b->d_awork);
+  cudaFree(b->d_slabs);
+  cudaFree(b->work3);
   for (auto &q : b->pending) {
     if (q.ev_main) cudaEventDestroy(q.ev_main);
     if (q.ev_io) cudaEventDestroy(q.ev_io);
@@ -450,7 +493,8 @@ int smaug_batch_destroy(smaug_batch *b) {
   for (int k = 0; k < 2; ++k) {
     if (b->st_tab[k]) cudaFreeHost(b->st_tab[k]);
     if (b->st_work[k]) cudaFreeHost(b->st_work[k]);
-    if (b->st_gwork[k]) cudaFreeHost(b->st_gwork[k]);
+    if (b->st_awork[k]) cudaFreeHost(b->st_awork[k]);
+    if (b->st_slabs[k]) cudaFreeHost(b->st_slabs[k]);
     if (b->st_ev[k]) cudaEventDestroy(b->st_ev[k]);
   }
   if (b->up_done) cudaEventDestroy(b->up_done);
@@ -647,7 +691,7 @@ int smaug_batch_step(smaug_batch *b, int nsteps) {
   if (b->nwork == 0) return SMAUG_OK;
   if (b->profile) {
     for (int i = 0; i < nsteps; ++i) enqueue_step(b, b->stream, true);
-    b->launches += (long long)kLaunchesPerStep * nsteps;
+    b->launches += (long long)launches_per_step(b) * nsteps;
     BK(cudaGetLastError());
     return SMAUG_OK;
   }
@@ -661,11 +705,11 @@ int smaug_batch_step(smaug_batch *b, int nsteps) {
   }
   for (int i = 0; i + kGraphSteps <= nsteps; i += kGraphSteps) {
     BK(cudaGraphLaunch(b->gk, b->stream));
-    b->launches += (long long)kLaunchesPerStep * kGraphSteps;
+    b->launches += (long long)launches_per_step(b) * kGraphSteps;
   }
   for (int i = 0; i < nsteps % kGraphSteps; ++i) {
     BK(cudaGraphLaunch(b->g1, b->stream));
-    b->launches += kLaunchesPerStep;
+    b->launches += launches_per_step(b);
   }
   return SMAUG_OK;
 }
@@ -832,10 +876,10 @@ int smaug_batch_tune(smaug_batch *b, int reps, int *variant_out, double *ms_out,
     if (rc != SMAUG_OK) return rc;
     if (b->nwork == 0) break;
     batch_go_kernel<<<(b->max_inst + 127) / 128, 128, 0, b->stream>>>(b->d_tab, b->max_inst);
-    smaug_batchk::launch_batch_stage(b->D, b->mixed, v, b->d_tab, b->d_work, b->nwork, 1, b->grid, b->stream);
+    launch_rk_stage(b, 1, b->stream);
     BK(cudaEventRecord(e0, b->stream));
     for (int r = 0; r < reps; ++r)
-      smaug_batchk::launch_batch_stage(b->D, b->mixed, v, b->d_tab, b->d_work, b->nwork, 1, b->grid, b->stream);
+      launch_rk_stage(b, 1, b->stream);
     BK(cudaEventRecord(e1, b->stream));
     BK(cudaEventSynchronize(e1));
     // a launch that the device refused (a configuration error, reported
@@ -847,7 +891,7 @@ int smaug_batch_tune(smaug_batch *b, int reps, int *variant_out, double *ms_out,
     float ms = 0.f;
     BK(cudaEventElapsedTime(&ms, e0, e1));
     ms /= reps;
-    b->launches += reps + 2;
+    b->launches += 1 + (long long)(reps + 1) * launches_per_rk_stage(b);
     if (ms_out && v < nms) ms_out[v] = ms;
     if (ms < best_ms) {
       best_ms = ms;

@@ -42,7 +42,11 @@ struct Run : SimPlan {
   // one simulation (so a simulation gives the same bits alone and in a batch)
   BatchInst *inst = nullptr;
   BatchInst h_inst{};
-  int ntiles = 0;
+  Plan3 plan3;  // 3-D: the slabs and items of a stage, their device lists and workspace
+  Slab3 *slabs = nullptr;
+  WorkItem *items = nullptr;
+  char *work3 = nullptr;
+  int ntiles = 0, sms = 148;
   int grid = 0;  // persistent grid of the batch stage kernel (blocks), at most ntiles
   int cur = 0;
   long long launches = 0;
@@ -111,20 +115,20 @@ void launch_stage(Run &r, const StageArgs &a) {
     else
       smaug_fast::launch_stage(r.D, r.mixed, a, r.geo, r.phys, r.stream);
   });
-  if (!r.exact) r.launches++;  // the tiled build's ghost pass
 }
 
 // RK stage k (1..4) of the production path: the batch stage kernel, one
 // block per tile of this simulation.
 void launch_rk_stage(Run &r, int k) {
   timed_launch(r, [&] {
-    smaug_batchk::launch_batch_stage(r.D, r.mixed, batch_default_variant(r.D, r.mixed), r.inst, nullptr, r.ntiles, k,
-                                     r.grid, r.stream);
+    const int v = batch_default_variant(r.D, r.mixed);
+    if (r.D == 2)
+      smaug_batchk::launch_batch_stage2(r.mixed, v, r.inst, nullptr, r.ntiles, k, r.grid, r.stream);
+    else
+      r.launches += smaug_batchk::launch_pass3(r.mixed, v, r.inst, r.slabs, r.items, r.plan3, k, r.grid, r.stream) - 1;
+    smaug_batchk::launch_batch_advance(r.D, r.mixed, r.inst, nullptr, advance_items(r.geo, r.D), k, r.sms, r.stream);
+    r.launches++;
   });
-  // its ghost pass: the ghost chunks of this simulation
-  const int nch = (int)((ghost_cells(r.geo, r.D) + 255) / 256);
-  smaug_batchk::launch_batch_ghost(r.D, r.mixed, r.inst, nullptr, nch, k, std::min(nch, 148 * 8), r.stream);
-  r.launches++;
 }
 
 // Describe the simulation to the batch stage kernel (production RK4 path).
@@ -149,11 +153,30 @@ cudaError_t run_upload_inst(Run &r) {
   }
   // a persistent grid, as a batch runs it: resident blocks on every SM, each
   // looping over tiles and keeping its maxima across them
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, dev);
   const int occ = std::max(1, smaug_batchk::batch_stage_occupancy(r.D, r.mixed, batch_default_variant(r.D, r.mixed)));
-  r.grid = std::min(r.ntiles, occ * sms);
+  r.grid = r.D == 2 ? std::min(r.ntiles, occ * r.sms) : occ * r.sms;
   return cudaMemcpyAsync(r.inst, &I, sizeof(BatchInst), cudaMemcpyHostToDevice, r.stream);
+}
+
+// The 3-D stage's plan, lists and workspace (allocated once, with the context).
+cudaError_t run_plan3(Run &r) {
+  if (r.D != 3 || !r.rk4 || r.exact) return cudaSuccess;
+  int t[3];
+  batch_tile_shape(3, batch_default_variant(3, r.mixed), t);
+  r.plan3.build({{0, r.geo}}, t, r.mixed);
+  cudaError_t e = cudaMalloc(&r.work3, r.plan3.bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&r.slabs, sizeof(Slab3) * r.plan3.slabs.size());
+  if (e == cudaSuccess) e = cudaMalloc(&r.items, sizeof(WorkItem) * r.plan3.items.size());
+  if (e != cudaSuccess) return e;
+  r.plan3.place(r.work3);
+  e = cudaMemcpyAsync(r.slabs, r.plan3.slabs.data(), sizeof(Slab3) * r.plan3.slabs.size(), cudaMemcpyHostToDevice,
+                      r.stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(r.items, r.plan3.items.data(), sizeof(WorkItem) * r.plan3.items.size(), cudaMemcpyHostToDevice,
+                        r.stream);
+  return e;
 }
 
 // A state is in r.W[0] (evolved) and r.bg: fill ghosts, reset scalars,
@@ -214,7 +237,7 @@ cudaError_t run_stage(Run &r, int k) {
   StageArgs a{};
   a.bg = r.bg;
   a.sc = r.sc;
-  if (r.mixed || (r.rk4 && !r.exact)) {
+  if (r.mixed || (r.rk4 && !r.exact && (r.D == 2 || r.work3))) {
     // production fourstep, FP64 or mixed (FP32 stage states: S1 = W + dt/2
     // L(W), S2 = W + dt/2 L(S1), S3 = W + dt L(S2), A = (S1 + 2 S2 + S3 -
     // 4 W)/3 accumulated stage by stage, W <- W + dt/6 L(S3) + A); the stage
@@ -316,6 +339,7 @@ int smaug_create(const smaug_params *prm, int device, smaug_ctx **out) {
   CK(cudaMalloc(&ctx->dxlast, fsz));
   CK(cudaMalloc(&r.sc, sizeof(DevScalars)));
   CK(cudaMalloc(&r.inst, sizeof(BatchInst)));
+  CK(run_plan3(r));
   {
     const size_t nl = (size_t)r.geo.n[0] + r.geo.n[1] + r.geo.n[2];
     std::vector<double> lines(nl);
@@ -348,6 +372,9 @@ int smaug_destroy(smaug_ctx *ctx) {
   cudaFree(ctx->dxlast);
   cudaFree(r.sc);
   cudaFree(r.inst);
+  cudaFree(r.work3);
+  cudaFree(r.slabs);
+  cudaFree(r.items);
   drop_graphs(r);
   for (auto e : ctx->ev) cudaEventDestroy(e);
   if (ctx->join) cudaEventDestroy(ctx->join);

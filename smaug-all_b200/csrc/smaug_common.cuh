@@ -154,13 +154,6 @@ __global__ void ghost_pass_kernel(double *w, int nw, Geo g, int D, int d) {
   }
 }
 
-// Ghost cells of a grid (a coordinate outside [2, n-3]).
-inline long long ghost_cells(const Geo &g, int D) {
-  long long in = 1;
-  for (int d = 0; d < D; ++d) in *= g.n[d] - 4;
-  return g.N - in;
-}
-
 // The ghost fill of a loaded state, used when a state is loaded
 // (iosmaug.cpp:786-794).
 void ghost_fill(double *w, int nw, const Geo &g, int D, cudaStream_t s) {

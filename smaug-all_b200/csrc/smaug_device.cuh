@@ -88,6 +88,8 @@ struct StageArgs {
   // an FP32 compensation (w32 + c32 carries ~48 bits), FP32 RK increment sum
   const float *in32;
   float *out32, *acc32, *w32, *c32;
+  double *src;         // the sources dL of the inner cells between the stage and the advance pass
+  float *src32;
   DevScalars *sc;
   int kind;            // FP64: 0 plain, 3 = RK stage 3, 4 = RK stage 4; mixed: RK stage 1..4
   int red_in, red_out; // reduction slots: cmax of `in`, maxima of `out`
@@ -288,13 +290,13 @@ __device__ __forceinline__ void visc_at(const Cell<D> &c, const Geo &g, long lon
 // from the host-computed factor lines, tdep = sin(2 pi t / P) or 1 (P = 0).
 // The driven momentum then gains h * vvz * (rho + rhob) of the stage output
 // (models/usersource.cu.spicule1:4-137, addsourceterms2).
+__device__ __forceinline__ double driver_tdep(const Phys &p, const DevScalars *sc, double tfrac) {
+  return p.drv_period > 0.0 ? sin(2.0 * 3.14159265358979323846 * (sc->t + tfrac * sc->dt) / p.drv_period) : 1.0;
+}
 template <int D>
-__device__ __forceinline__ double driver_vvz(const Geo &g, const Phys &p, const DevScalars *sc, double tfrac,
-                                             const int *c) {
+__device__ __forceinline__ double driver_vvz(const Geo &g, const Phys &p, double tdep, const int *c) {
   double f = g.drvf[1][c[1]] * g.drvf[0][c[0]];
   if (D == 3) f = f * g.drvf[2][c[2]];
-  double tdep = 1.0;
-  if (p.drv_period > 0.0) tdep = sin(2.0 * 3.14159265358979323846 * (sc->t + tfrac * sc->dt) / p.drv_period);
   return p.drv_amp * f * tdep;
 }
 

@@ -50,45 +50,42 @@ __device__ __forceinline__ double grad3d_at(const Cell<D> &C, const Geo &g, cons
   return grad;
 }
 
-// Block-wide max of v[0..5] then one atomic per value into r.
-template <int NV>
-__device__ __forceinline__ void block_max_flush(double *v, Reduce *r) {
-  __shared__ double sm[NV][32];
-  const int lane = (threadIdx.x + threadIdx.y * blockDim.x + threadIdx.z * blockDim.x * blockDim.y) & 31;
-  const int warp = (threadIdx.x + threadIdx.y * blockDim.x + threadIdx.z * blockDim.x * blockDim.y) >> 5;
+// Maxima over a warp of non-negative values or NaN (kept: its bit pattern
+// compares above every number's); FP32 in one instruction on the bit pattern.
+__device__ __forceinline__ double warp_max(double x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double y = __shfl_xor_sync(0xffffffffu, x, o);
+    x = (y > x || y != y) ? y : x;
+  }
+  return x;
+}
+__device__ __forceinline__ float warp_max(float x) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x)));
+}
+
+// Block-wide maxima of v[0 .. NV-1], then one atomic per value into r.v[K0 ..]
+// (FP32 values widened exactly): warps first, then one thread per value over
+// the warps.
+template <int K0, int NV, typename T>
+__device__ __forceinline__ void block_max_flush(const T *v, Reduce *r) {
+  __shared__ T sm[NV][32];
+  const int t = threadIdx.x + threadIdx.y * blockDim.x + threadIdx.z * blockDim.x * blockDim.y;
   const int nwarp = (blockDim.x * blockDim.y * blockDim.z + 31) >> 5;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    double x = v[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      double y = __shfl_xor_sync(0xffffffffu, x, o);
-      x = (y > x || y != y) ? y : x;
-    }
-    if (lane == 0) sm[k][warp] = x;
+    const T x = warp_max(v[k]);
+    if ((t & 31) == 0) sm[k][t >> 5] = x;
   }
   __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double x = lane < nwarp ? sm[k][lane] : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        double y = __shfl_xor_sync(0xffffffffu, x, o);
-        x = (y > x || y != y) ? y : x;
-      }
-      if (lane == 0 && x != 0.0) atomic_max_nonneg(&r->v[k], x);
+  if (t < NV) {
+    T x = sm[t][0];
+    for (int w = 1; w < nwarp; ++w) {
+      const T y = sm[t][w];
+      x = (y > x || y != y) ? y : x;
     }
+    if (x != T(0)) atomic_max_nonneg(&r->v[K0 + t], (double)x);
   }
-}
-
-// The same for FP32 running maxima (widened exactly to FP64).
-template <int NV>
-__device__ __forceinline__ void block_max_flush(const float *v, Reduce *r) {
-  double w[NV];
-#pragma unroll
-  for (int k = 0; k < NV; ++k) w[k] = (double)v[k];
-  block_max_flush<NV>(w, r);
 }
 
 // Coordinates along d that take the value of inner coordinate x once the
@@ -405,7 +402,7 @@ __global__ void __launch_bounds__(kBX *kBY) stage_kernel(StageArgs a, Geo g, Phy
 
     // ---- momentum driver on the stage output (usersource.cu.spicule1:4-137)
     if (p.drv_on) {
-      const double vvz = driver_vvz<D>(g, p, a.sc, a.tfrac, c);
+      const double vvz = driver_vvz<D>(g, p, driver_tdep(p, a.sc, a.tfrac), c);
       const double rb = __ldg(a.bg + (long long)(L::RHOB - NW) * N + idx);
 #pragma unroll
       for (int k = 0; k < D; ++k)
@@ -453,7 +450,7 @@ __global__ void __launch_bounds__(kBX *kBY) stage_kernel(StageArgs a, Geo g, Phy
           reduce_cell<D>(g, p, ov, bgv, j, red);
         }
   }
-  block_max_flush<6>(red, &a.sc->red[a.red_out]);
+  block_max_flush<0, 6>(red, &a.sc->red[a.red_out]);
 }
 
 // Maxima over all cells of a state (used once after the state is loaded);
@@ -475,7 +472,7 @@ __global__ void reduce_state_kernel(const double *w, const double *bg, Geo g, Ph
     for (int b = 0; b < NB; ++b) bgv[b] = bg[(long long)b * g.N + j];
     reduce_cell<D>(g, p, o, bgv, j, red);
   }
-  block_max_flush<6>(red, r);
+  block_max_flush<0, 6>(red, r);
 }
 
 }  // namespace SMAUG_NS

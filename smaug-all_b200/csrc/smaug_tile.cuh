@@ -69,6 +69,27 @@ __device__ __forceinline__ float vabs(float a) { return fabsf(a); }
 // a * b + c with one rounding (never left to contraction)
 __device__ __forceinline__ double vfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+// Conversions between the stencil type and FP64 (none when it is FP64).  The
+// plain casts of the -ftz=true build flush subnormals around the conversion
+// (a multiply before it, a compare and a select after it), which in the mixed
+// kernels was a tenth of all instructions; the FP32 arithmetic that reads a
+// converted value flushes it anyway.
+__device__ __forceinline__ double dbl(double x) { return x; }
+__device__ __forceinline__ double dbl(float x) {
+  double r;
+  asm("cvt.f64.f32 %0, %1;" : "=d"(r) : "f"(x));
+  return r;
+}
+template <typename T>
+__device__ __forceinline__ T num(double x) {
+  if constexpr (sizeof(T) == sizeof(float)) {
+    float r;
+    asm("cvt.rn.f32.f64 %0, %1;" : "=f"(r) : "d"(x));
+    return r;
+  } else {
+    return x;
+  }
+}
 // The hyperviscosity ratio a / b (b > 0): IEEE division in FP64; in FP32 the
 // reciprocal-based quotient (within 2 ulp), the ratio being a limiter weight.
 __device__ __forceinline__ double vratio(double a, double b) { return a / b; }
@@ -89,11 +110,11 @@ struct CellT {
   long long N;
   // field f at cell i in the stencil type
   __device__ __forceinline__ T v(int f, long long i) const {
-    return f < Lay<D>::NW ? __ldg(in + fo32(f, N, i)) : (T)__ldg(bg + fo32(f - Lay<D>::NW, N, i));
+    return f < Lay<D>::NW ? __ldg(in + fo32(f, N, i)) : num<T>(__ldg(bg + fo32(f - Lay<D>::NW, N, i)));
   }
   // field f at cell i in FP64
   __device__ __forceinline__ double vd(int f, long long i) const {
-    return f < Lay<D>::NW ? (double)__ldg(in + fo32(f, N, i)) : __ldg(bg + fo32(f - Lay<D>::NW, N, i));
+    return f < Lay<D>::NW ? dbl(__ldg(in + fo32(f, N, i))) : __ldg(bg + fo32(f - Lay<D>::NW, N, i));
   }
 };
 
@@ -113,9 +134,9 @@ template <int D, typename T>
 __device__ __forceinline__ void fluxes_fast(const CellT<D, T> &c, long long i, int dir, double gam, bool bgb, T *F) {
   using L = Lay<D>;
   const T rho = c.v(L::RHO, i);
-  const double rt = (double)rho + c.vd(L::RHOB, i);
+  const double rt = dbl(rho) + c.vd(L::RHOB, i);
   const double irtd = __drcp_rn(rt);
-  const T irt = (T)irtd;
+  const T irt = num<T>(irtd);
   T m[D], b[D], bb[D];
 #pragma unroll
   for (int k = 0; k < D; ++k) {
@@ -128,13 +149,13 @@ __device__ __forceinline__ void fluxes_fast(const CellT<D, T> &c, long long i, i
   T bbm = 0, bm = 0;
 #pragma unroll
   for (int k = 0; k < D; ++k) {
-    bbb += (double)b[k] * (double)bb[k];
-    b2 += (double)b[k] * (double)b[k];
-    m2 += (double)m[k] * (double)m[k];
+    bbb += dbl(b[k]) * dbl(bb[k]);
+    b2 += dbl(b[k]) * dbl(b[k]);
+    m2 += dbl(m[k]) * dbl(m[k]);
     bbm += bb[k] * m[k];
     bm += b[k] * m[k];
   }
-  const T pt = (T)((gam - 1.0) * ((double)e - 0.5 * m2 * irtd) - (gam - 2.0) * (bbb + 0.5 * b2));
+  const T pt = num<T>((gam - 1.0) * (dbl(e) - 0.5 * m2 * irtd) - (gam - 2.0) * (bbb + 0.5 * b2));
   const T md = m[dir], vd = md * irt;
   const T bd = b[dir], bbd = bb[dir];
   F[L::RHO] = md;
@@ -157,18 +178,18 @@ template <int D, typename T>
 __device__ __forceinline__ void q_all(const CellT<D, T> &c, long long i, int d, T *q) {
   using L = Lay<D>;
   const T rho = c.v(L::RHO, i);
-  const double irtd = __drcp_rn((double)rho + c.vd(L::RHOB, i));
-  const T irt = (T)irtd;
+  const double irtd = __drcp_rn(dbl(rho) + c.vd(L::RHOB, i));
+  const T irt = num<T>(irtd);
   double b2 = 0, m2 = 0;
   q[0] = rho;
 #pragma unroll
   for (int k = 0; k < D; ++k) {
     const T m = c.v(L::M0 + k, i), b = c.v(L::B0 + k, i);
-    b2 += (double)b * (double)b;
-    m2 += (double)m * (double)m;
+    b2 += dbl(b) * dbl(b);
+    m2 += dbl(m) * dbl(m);
     q[2 + k] = m * irt;
   }
-  q[1] = (T)(c.vd(L::EN, i) - 0.5 * (b2 + m2 * irtd));
+  q[1] = num<T>(c.vd(L::EN, i) - 0.5 * (b2 + m2 * irtd));
   int s = 2 + D;
 #pragma unroll
   for (int f = 0; f < D; ++f)
@@ -199,11 +220,11 @@ template <int D>
 __device__ __forceinline__ void reduce_cell_mixed(const Geo &g, const Phys &p, const float *o, const double *b,
                                                   long long idx, float *r) {
   using L = Lay<D>;
-  const float irt = __frcp_rn((float)((double)o[L::RHO] + b[1]));
+  const float irt = __frcp_rn(num<float>(dbl(o[L::RHO]) + b[1]));
   float m2 = 0.0f, b2 = 0.0f, bbb = 0.0f, bb2 = 0.0f;
 #pragma unroll
   for (int k = 0; k < D; ++k) {
-    const float m = o[L::M0 + k], bf = o[L::B0 + k], bb = (float)b[2 + k];
+    const float m = o[L::M0 + k], bf = o[L::B0 + k], bb = num<float>(b[2 + k]);
     m2 = __fmaf_rn(m, m, m2);
     b2 = __fmaf_rn(bf, bf, b2);
     bbb = __fmaf_rn(bb, bf, bbb);
@@ -215,16 +236,16 @@ __device__ __forceinline__ void reduce_cell_mixed(const Geo &g, const Phys &p, c
                                        __fmul_rn(0.5f, b2)), bbb);
   const float pk = __fmul_rn(gm1, ek);
   // c_s^2 = gamma (p_k + (gamma-1)(e_b - B_b^2/2)) / rho_t
-  const float pbg = __fmul_rn(gm1, __fsub_rn((float)b[0], __fmul_rn(0.5f, bb2)));
+  const float pbg = __fmul_rn(gm1, __fsub_rn(num<float>(b[0]), __fmul_rn(0.5f, bb2)));
   const float cs2 = __fmul_rn(__fmul_rn(gam, __fadd_rn(pk, pbg)), irt);
   const float cf = __fadd_rn(__fmul_rn(__fadd_rn(__fadd_rn(b2, bb2), __fmul_rn(2.0f, bbb)), irt), cs2);
   {
     constexpr float kBelow = 1.0f - 1e-5f;
-    const float rdx = __fdividef(1.0f, (float)__ldg(g.dxlast + idx));
+    const float rdx = __fdividef(1.0f, num<float>(__ldg(g.dxlast + idx)));
     bool need = false;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      const float bd = (float)(b[2 + d] + (double)o[L::B0 + d]);
+      const float bd = num<float>(b[2 + d] + dbl(o[L::B0 + d]));
       const float disc =
           __fsub_rn(__fmul_rn(cf, cf), __fmul_rn(__fmul_rn(__fmul_rn(4.0f, cs2), __fmul_rn(bd, bd)), irt));
       const float cfi = __fmul_rn(0.5f, __fadd_rn(cf, sqrt_approx(fmaxf(disc, 0.0f))));
@@ -240,117 +261,260 @@ __device__ __forceinline__ void reduce_cell_mixed(const Geo &g, const Phys &p, c
   }
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    const float bd = (float)(b[2 + d] + (double)o[L::B0 + d]);
+    const float bd = num<float>(b[2 + d] + dbl(o[L::B0 + d]));
     const float disc = __fsub_rn(__fmul_rn(cf, cf), __fmul_rn(__fmul_rn(__fmul_rn(4.0f, cs2), __fmul_rn(bd, bd)), irt));
     const float cfi = __fmul_rn(0.5f, __fadd_rn(cf, __fsqrt_rn(fmaxf(disc, 0.0f))));
     const float cff = __fadd_rn(__fsqrt_rn(cfi), fabsf(__fmul_rn(o[L::M0 + d], irt)));
     if (cff > r[d] || cff != cff) r[d] = cff;
     if (d == D - 1) {
-      const float cour = __fmul_rn(cff, __frcp_rn((float)__ldg(g.dxlast + idx)));
+      const float cour = __fmul_rn(cff, __frcp_rn(num<float>(__ldg(g.dxlast + idx))));
       if (cour > r[3] || cour != cour) r[3] = cour;
       if (idx >= g.K && (cour > r[4] || cour != cour)) r[4] = cour;
     }
   }
 }
 
-// The end of a stage for one cell: the stage output base + h dL with the
-// driver, the RK combination of the stage, the write of the cell and the
-// wave-speed / viscosity maxima, taken into the
-// thread's running maxima red[6] (in the stencil type: FP32 values in the
-// mixed path; the caller flushes them to the simulation's reduction slot).
+// reduce_cell (FP64) behind a screen, as in reduce_cell_mixed: the speeds with
+// one reciprocal of rho_t, hardware-approximated square roots and metric
+// reciprocal lie within 1e-5 of the exact ones (the terms under the roots carry
+// a few roundings of cf^2, at most 1e-7 of cf after the root; the
+// approximations themselves 2^-20), so a cell that stays more than 1e-5 below
+// the running maxima cannot raise them.  Any other cell, a NaN included, takes
+// reduce_cell: the maxima keep their bits.  (Nine divisions and six square
+// roots in software per 3-D cell otherwise.)
+__device__ __forceinline__ double rsqrt_approx(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  return r;
+}
+__device__ __forceinline__ double rcp_approx(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  return r;
+}
+template <int D>
+__device__ __forceinline__ void reduce_cell_screened(const Geo &g, const Phys &p, const double *o, const double *b,
+                                                     long long idx, double *r) {
+  using L = Lay<D>;
+  const double irt = __drcp_rn(o[L::RHO] + b[1]);
+  double m2 = 0, b2 = 0, bbb = 0, bb2 = 0;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    m2 += o[L::M0 + k] * o[L::M0 + k];
+    b2 += o[L::B0 + k] * o[L::B0 + k];
+    bbb += b[2 + k] * o[L::B0 + k];
+    bb2 += b[2 + k] * b[2 + k];
+  }
+  const double pk = (p.gamma - 1) * (o[L::EN] - 0.5 * m2 * irt - 0.5 * b2 - bbb);
+  const double cs2 = p.gamma * (pk + (p.gamma - 1) * (b[0] - 0.5 * bb2)) * irt;
+  const double cf = (b2 + bb2 + 2.0 * bbb) * irt + cs2;
+  constexpr double kBelow = 1.0 - 1e-5;
+  const double rdx = rcp_approx(__ldg(g.dxlast + idx));
+  bool need = false;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const double bd = b[2 + d] + o[L::B0 + d];
+    const double disc = cf * cf - 4.0 * cs2 * (bd * bd) * irt;
+    const double cfi = 0.5 * (cf + (disc > 0.0 ? disc * rsqrt_approx(disc) : disc));
+    const double cff = cfi * rsqrt_approx(cfi) + fabs(o[L::M0 + d] * irt);
+    need |= !(cff < r[d] * kBelow);
+    if (d == D - 1) {
+      const double cour = cff * rdx;
+      need |= !(cour < r[3] * kBelow);
+      if (idx >= g.K) need |= !(cour < r[4] * kBelow);
+    }
+  }
+  if (need) reduce_cell<D>(g, p, o, b, idx, r);
+}
+
+// Loads and stores of the advance pass: every value is touched once, so it
+// passes by L1 (and the instructions are global ones: the buffer pointers come
+// from a table in memory, where the compiler does not know their space).
+__device__ __forceinline__ float ldq(const float *p) { return __ldcg(p); }
+__device__ __forceinline__ double ldq(const double *p) { return __ldcg(p); }
+__device__ __forceinline__ void stq(float *p, float v) { __stcg(p, v); }
+__device__ __forceinline__ void stq(double *p, double v) { __stcg(p, v); }
+
+// The sources dL of one inner cell on their way from the stage kernel to the
+// advance pass.
 template <int D, typename T>
-__device__ __forceinline__ void stage_epilogue(const StageArgs &a, const Geo &g, const Phys &p, const CellT<D, T> &C,
-                                               const int *c, bool active, long long idx, double h, const T *dL,
-                                               T numax, T *red) {
+__device__ __forceinline__ void store_sources(const StageArgs &a, const Geo &g, long long idx, const T *dL) {
+  T *o = sizeof(T) == sizeof(float) ? (T *)(void *)a.src32 : (T *)(void *)a.src;
+#pragma unroll
+  for (int f = 0; f < Lay<D>::NW; ++f) stq(o + fo32(f, g.N, idx), dL[f]);
+}
+template <int D, typename T>
+__device__ __forceinline__ void load_sources(const StageArgs &a, const Geo &g, long long idx, T *dL) {
+  const T *o = sizeof(T) == sizeof(float) ? (const T *)(const void *)a.src32 : (const T *)(const void *)a.src;
+#pragma unroll
+  for (int f = 0; f < Lay<D>::NW; ++f) dL[f] = ldq(o + fo32(f, g.N, idx));
+}
+
+// Wave-speed maxima of the state v (of the inner cell or one of its images)
+// at cell j, with that cell's backgrounds (e_b and B_b are zero everywhere
+// without an energy background: only rho_b is read then).
+template <int D, typename T>
+__device__ __forceinline__ void reduce_at(const StageArgs &a, const Geo &g, const Phys &p, const T *v, long long j,
+                                          T *red) {
   using L = Lay<D>;
   constexpr int NW = L::NW, NB = L::NVAR - NW;
+  double bgv[NB];
+#pragma unroll
+  for (int b = 0; b < NB; ++b)
+    bgv[b] = (b == L::RHOB - NW || p.has_bgb) ? __ldg(a.bg + fo32(b, g.N, j)) : 0.0;
+  if constexpr (sizeof(T) == sizeof(float))
+    reduce_cell_mixed<D>(g, p, v, bgv, j, red);
+  else
+    reduce_cell_screened<D>(g, p, v, bgv, j, red);
+}
+
+// The end of a stage for one inner cell: the stage output base + h dL with the
+// driver, the RK combination of the stage (KIND: StageArgs::kind), the write of
+// the cell and of its ghost images (the reference's boundary pass after each
+// step, iosmaug.cpp:1157-1166; a stage reads no buffer that it writes beyond
+// the cell itself), and the wave-speed maxima of all of them (the reference's
+// c_max covers the ghosts), taken into the thread's running maxima red[5] (in
+// the stencil type: FP32 values in the mixed path; the caller flushes them to
+// the simulation's reduction slot).  Everything the cell reads is loaded
+// before its first store: a load behind a store to another buffer waits for it
+// (the buffers may alias as far as the compiler knows), and field by field
+// that was one memory latency per field.
+template <int D, typename T, int KIND>
+__device__ __forceinline__ void advance_cell(const StageArgs &a, const Geo &g, const Phys &p, const int *c,
+                                             long long idx, double h, double tdep, const T *dL, T *red) {
+  using L = Lay<D>;
+  constexpr int NW = L::NW;
   constexpr bool MIXED = sizeof(T) == sizeof(float);
-  if (numax > red[5] || numax != numax) red[5] = numax;
-  if (active) {
-    double o[NW];
-    float hi[NW], lo[NW];
-    if (!MIXED) {
+  T o[NW];   // the stage output (mixed: FP32 value)
+  T lo[NW];  // what goes with it: the sum so far, in mixed stage 4 the compensation
+  if constexpr (!MIXED) {
+    double bv[NW], iv[NW];
 #pragma unroll
-      for (int f = 0; f < NW; ++f) o[f] = a.base[fo32(f, g.N, idx)] + h * (double)dL[f];
-      if (p.drv_on) {  // momentum driver on the stage output (before the RK combination)
-        const double vvz = driver_vvz<D>(g, p, a.sc, a.tfrac, c);
-        const double rb = __ldg(a.bg + (long long)(L::RHOB - NW) * g.N + idx);
-        // (unrolled compare: a runtime index would push o to local memory)
+    for (int f = 0; f < NW; ++f) bv[f] = ldq(a.base + fo32(f, g.N, idx));
+    if (KIND >= 3) {
 #pragma unroll
-        for (int k = 0; k < D; ++k)
-          if (k == p.drv_dir) o[L::M0 + k] = o[L::M0 + k] + h * vvz * (o[L::RHO] + rb);
-      }
-      if (a.kind == 3) {
-#pragma unroll
-        for (int f = 0; f < NW; ++f) {
-          const unsigned j = fo32(f, g.N, idx);
-          a.acc[j] = (a.acc[j] + 2.0 * C.vd(f, idx) + o[f] - 4.0 * a.base[j]) * (1.0 / 3.0);
-        }
-      } else if (a.kind == 4) {
-#pragma unroll
-        for (int f = 0; f < NW; ++f) o[f] += a.acc[fo32(f, g.N, idx)];
-      }
-    } else {
-      // RK4 in increment form, W = w32 + c32:
-      //   stages k = 1..3: S_k = W + h_k L_k (FP32), A += c_k h_k L_k with
-      //   c = 1/3, 2/3, 1/3, so A = (S1 + 2 S2 + S3 - 4 W) / 3 as the FP64 path;
-      //   stage 4: W <- W + h_4 L_4 + A, kept as value + compensation.
-      // Stages 1..3 round to FP32 anyway, so they take the base without c32.
-      // momentum driver with the stage output's density, added to the
-      // increment of m along drv_dir (dm = 0 without a driver)
-      double dm = 0.0;
-      int dm_f = -1;
-      if (p.drv_on) {
-        const double wr = a.kind == 4 ? (double)a.w32[idx] + (double)a.c32[idx] : (double)a.w32[idx];
-        const double rb = __ldg(a.bg + (long long)(L::RHOB - NW) * g.N + idx);
-        dm = h * driver_vvz<D>(g, p, a.sc, a.tfrac, c) * ((wr + h * (double)dL[L::RHO]) + rb);
-        dm_f = L::M0 + p.drv_dir;
-      }
-#pragma unroll
-      for (int f = 0; f < NW; ++f) {
-        const unsigned j = fo32(f, g.N, idx);
-        double inc = h * (double)dL[f];
-        if (f == dm_f) inc += dm;
-        if (a.kind == 4) {
-          const double wn = ((double)a.w32[j] + (double)a.c32[j]) + (inc + (double)a.acc32[j]);
-          hi[f] = (float)wn;
-          lo[f] = (float)(wn - (double)hi[f]);
-        } else {
-          hi[f] = (float)((double)a.w32[j] + inc);
-          const double prev = a.kind == 1 ? 0.0 : (double)a.acc32[j];
-          a.acc32[j] = (float)(prev + (a.kind == 2 ? 2.0 : 1.0) * (1.0 / 3.0) * inc);
-        }
-      }
+      for (int f = 0; f < NW; ++f) lo[f] = ldq(a.acc + fo32(f, g.N, idx));
     }
-    // the cell (its ghost images are written by the ghost pass that follows
-    // every stage: ghost_cell below)
-    {
-      const unsigned j = (unsigned)idx;
-      if (!MIXED) {
+    if (KIND == 3) {
 #pragma unroll
-        for (int f = 0; f < NW; ++f) a.out[fo32(f, g.N, j)] = o[f];
-      } else if (a.kind == 4) {
+      for (int f = 0; f < NW; ++f) iv[f] = ldq(a.in + fo32(f, g.N, idx));
+    }
 #pragma unroll
-        for (int f = 0; f < NW; ++f) {
-          a.w32[fo32(f, g.N, j)] = hi[f];
-          a.c32[fo32(f, g.N, j)] = lo[f];
-        }
+    for (int f = 0; f < NW; ++f) o[f] = bv[f] + h * dL[f];
+    if (p.drv_on) {  // momentum driver on the stage output (before the RK combination)
+      const double vvz = driver_vvz<D>(g, p, tdep, c);
+      const double rb = __ldg(a.bg + (long long)(L::RHOB - NW) * g.N + idx);
+      // (unrolled compare: a runtime index would push o to local memory)
+#pragma unroll
+      for (int k = 0; k < D; ++k)
+        if (k == p.drv_dir) o[L::M0 + k] = o[L::M0 + k] + h * vvz * (o[L::RHO] + rb);
+    }
+    if (KIND == 3) {
+#pragma unroll
+      for (int f = 0; f < NW; ++f)
+        stq(a.acc + fo32(f, g.N, idx), (lo[f] + 2.0 * iv[f] + o[f] - 4.0 * bv[f]) * (1.0 / 3.0));
+    } else if (KIND == 4) {
+#pragma unroll
+      for (int f = 0; f < NW; ++f) o[f] += lo[f];
+    }
+  } else {
+    // RK4 in increment form, W = w32 + c32:
+    //   stages k = 1..3: S_k = W + h_k L_k (FP32), A += c_k h_k L_k with
+    //   c = 1/3, 2/3, 1/3, so A = (S1 + 2 S2 + S3 - 4 W) / 3 as the FP64 path;
+    //   stage 4: W <- W + h_4 L_4 + A, kept as value + compensation.
+    // Stages 1..3 round to FP32 anyway, so they take the base without c32.
+    float wv[NW], cv[NW], av[NW];
+#pragma unroll
+    for (int f = 0; f < NW; ++f) wv[f] = ldq(a.w32 + fo32(f, g.N, idx));
+    if (KIND != 1) {
+#pragma unroll
+      for (int f = 0; f < NW; ++f) av[f] = ldq(a.acc32 + fo32(f, g.N, idx));
+    }
+    if (KIND == 4) {
+#pragma unroll
+      for (int f = 0; f < NW; ++f) cv[f] = ldq(a.c32 + fo32(f, g.N, idx));
+    }
+    // momentum driver with the stage output's density, added to the
+    // increment of m along drv_dir (dm = 0 without a driver)
+    double dm = 0.0;
+    int dm_f = -1;
+    if (p.drv_on) {
+      const double wr = KIND == 4 ? dbl(wv[0]) + dbl(cv[0]) : dbl(wv[0]);
+      const double rb = __ldg(a.bg + (long long)(L::RHOB - NW) * g.N + idx);
+      dm = h * driver_vvz<D>(g, p, tdep, c) * ((wr + h * dbl(dL[L::RHO])) + rb);
+      dm_f = L::M0 + p.drv_dir;
+    }
+#pragma unroll
+    for (int f = 0; f < NW; ++f) {
+      double inc = h * dbl(dL[f]);
+      if (f == dm_f) inc += dm;
+      if (KIND == 4) {
+        const double wn = (dbl(wv[f]) + dbl(cv[f])) + (inc + dbl(av[f]));
+        o[f] = num<float>(wn);
+        lo[f] = num<float>(wn - dbl(o[f]));
       } else {
-#pragma unroll
-        for (int f = 0; f < NW; ++f) a.out32[fo32(f, g.N, j)] = hi[f];
+        o[f] = num<float>(dbl(wv[f]) + inc);
+        const float sum = num<float>((KIND == 1 ? 0.0 : dbl(av[f])) + (KIND == 2 ? 2.0 : 1.0) * (1.0 / 3.0) * inc);
+        stq(a.acc32 + fo32(f, g.N, idx), sum);
       }
     }
-    // backgrounds (e_b and B_b are zero everywhere without an energy
-    // background: only rho_b is read then), then the maxima
-    double bgv[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-      bgv[b] = (b == L::RHOB - NW || p.has_bgb) ? __ldg(a.bg + fo32(b, g.N, (unsigned)idx)) : 0.0;
-    if constexpr (MIXED)
-      reduce_cell_mixed<D>(g, p, hi, bgv, idx, red);  // what the next stage reads
-    else
-      reduce_cell<D>(g, p, o, bgv, idx, red);
   }
+  // the cell (image 0) and its ghost images, all of cells within four cells of
+  // an end (images(): the rules of every direction composed)
+  bool near = false;
+#pragma unroll
+  for (int d = 0; d < D; ++d) near |= c[d] < 5 || c[d] > g.n[d] - 6;
+  int n0 = 1, n1 = 1, n2 = 1;
+  int xa = 0, xb = 0, ya = 0, yb = 0, za = 0, zb = 0;  // image coordinates per dimension
+  unsigned g0 = 0, g1 = 0, g2 = 0;
+  if (near) {
+    int x[3];
+    n0 = images<D>(g, 0, c[0], x, &g0);
+    xa = x[1];
+    xb = x[2];
+    n1 = images<D>(g, 1, c[1], x, &g1);
+    ya = x[1];
+    yb = x[2];
+    if (D == 3) {
+      n2 = images<D>(g, D - 1, c[D - 1], x, &g2);
+      za = x[1];
+      zb = x[2];
+    }
+  }
+  const int count = n0 * n1 * n2;
+  long long j = idx;
+  unsigned neg = 0;
+#pragma unroll 1
+  for (int k = 0;;) {
+    T v[NW];
+    T *w = MIXED ? (T *)(void *)(KIND == 4 ? a.w32 : a.out32) : (T *)(void *)a.out;
+#pragma unroll
+    for (int f = 0; f < NW; ++f) {
+      const unsigned q = fo32(f, g.N, j);
+      const bool m = (neg >> f) & 1u;
+      v[f] = m ? -o[f] : o[f];
+      stq(w + q, v[f]);
+      if (MIXED && KIND == 4) stq(a.c32 + q, m ? -(float)lo[f] : (float)lo[f]);
+    }
+    reduce_at<D, T>(a, g, p, v, j, red);  // what the next stage reads
+    if (++k >= count) break;
+    const int i0 = k % n0, r = k / n0, i1 = r % n1, i2 = r / n1;
+    j = (i0 == 0 ? c[0] : i0 == 1 ? xa : xb) + (i1 == 0 ? c[1] : i1 == 1 ? ya : yb) * g.st[1] +
+        (D == 3 ? (i2 == 0 ? c[2] : i2 == 1 ? za : zb) * g.st[2] : 0);
+    neg = (i0 ? g0 : 0u) ^ (i1 ? g1 : 0u) ^ (i2 ? g2 : 0u);
+  }
+}
+// The same with the kind at run time (single-step runs).
+template <int D, typename T>
+__device__ __forceinline__ void advance_cell_any(const StageArgs &a, const Geo &g, const Phys &p, const int *c,
+                                                 long long idx, double h, const T *dL, T *red) {
+  const double tdep = p.drv_on ? driver_tdep(p, a.sc, a.tfrac) : 0.0;
+  if (a.kind == 3)
+    advance_cell<D, T, 3>(a, g, p, c, idx, h, tdep, dL, red);
+  else if (a.kind == 4)
+    advance_cell<D, T, 4>(a, g, p, c, idx, h, tdep, dL, red);
+  else
+    advance_cell<D, T, 0>(a, g, p, c, idx, h, tdep, dL, red);
 }
 
 // Divergence-of-B source terms at an inner cell (cudivb, divb.cu:165-336 with
@@ -376,9 +540,9 @@ __device__ __forceinline__ void divb_sources(const CellT<2, T> &C, const Geo &g,
       const long long j = idx + (k < 2 ? k - 2 : k - 1) * s;
       b[k] = C.v(L::B0 + d, j) + (p.has_bgb ? C.v(L::BB0 + d, j) : T(0));
     }
-    divb += ((T)8 * (b[2] - b[1]) - (b[3] - b[0])) * (T)(1.0 / (12.0 * p.dxs[d]));
+    divb += ((T)8 * (b[2] - b[1]) - (b[3] - b[0])) * num<T>(1.0 / (12.0 * p.dxs[d]));
   }
-  const T irt = (T)(1.0 / (C.vd(L::RHO, idx) + C.vd(L::RHOB, idx)));
+  const T irt = num<T>(1.0 / (C.vd(L::RHO, idx) + C.vd(L::RHOB, idx)));
   T bdotv = 0;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
@@ -393,146 +557,10 @@ __device__ __forceinline__ void divb_sources(const CellT<2, T> &C, const Geo &g,
   dL[L::EN] += divb * bdotv * irt;
 }
 
-// ------------------------------------------------------------ the ghost pass
-// After every stage the ghost cells of the stage output are filled from the
-// inner cells just written (the reference's boundary pass after each step,
-// iosmaug.cpp:1157-1166), and their wave speeds join the stage's maxima (the
-// reference's c_max covers the ghosts).  Each ghost cell gathers its value:
-// from the last direction whose pass writes it, back along the chain of
-// sources (smaug_device.cuh) to an inner cell, negating the fields of the
-// asymm rules on the way; a chain that meets a fixed pass ends at a cell that
-// keeps its loaded value, so the ghost is left alone.
-
-// Ghost cells of a grid: the cells with a coordinate outside [2, n-3].
-template <int D>
-__host__ __device__ inline long long ghost_count(const Geo &g) {
-  long long in = 1;
-  for (int d = 0; d < D; ++d) in *= g.n[d] - 4;
-  return g.N - in;
-}
-
-// Coordinates of ghost k: first the four ghost rows (2-D) or planes (3-D) of
-// the last dim, then, for each inner coordinate of the last dim, the ring of
-// the lower dims.
-template <int D>
-__device__ __forceinline__ void ghost_coords(const Geo &g, long long k, int *c) {
-  const int n0 = g.n[0], n1 = g.n[1];
-  if (D == 2) {
-    if (k < 4LL * n0) {
-      const int r = (int)(k / n0);
-      c[0] = (int)(k - (long long)r * n0);
-      c[1] = r < 2 ? r : n1 - 4 + r;
-    } else {
-      const long long q = k - 4LL * n0;
-      const int r = (int)(q & 3);
-      c[1] = 2 + (int)(q >> 2);
-      c[0] = r < 2 ? r : n0 - 4 + r;
-    }
-    c[2] = 0;
-  } else {
-    const long long pl = (long long)n0 * n1;
-    const int n2 = g.n[2];
-    if (k < 4 * pl) {
-      const int r = (int)(k / pl);
-      const long long q = k - r * pl;
-      c[2] = r < 2 ? r : n2 - 4 + r;
-      c[1] = (int)(q / n0);
-      c[0] = (int)(q - (long long)c[1] * n0);
-    } else {
-      const long long ring = pl - (long long)(n0 - 4) * (n1 - 4);
-      const long long q0 = k - 4 * pl;
-      const long long z = q0 / ring;
-      const long long q = q0 - z * ring;
-      c[2] = 2 + (int)z;
-      if (q < 4LL * n0) {
-        const int r = (int)(q / n0);
-        c[0] = (int)(q - (long long)r * n0);
-        c[1] = r < 2 ? r : n1 - 4 + r;
-      } else {
-        const long long u = q - 4LL * n0;
-        const int r = (int)(u & 3);
-        c[1] = 2 + (int)(u >> 2);
-        c[0] = r < 2 ? r : n0 - 4 + r;
-      }
-    }
-  }
-}
-
-// Fill ghost k of the stage output and take its wave speeds into red.
-template <int D, typename T>
-__device__ __forceinline__ void ghost_cell(const StageArgs &a, const Geo &g, const Phys &p, long long k, T *red) {
-  using L = Lay<D>;
-  constexpr int NW = L::NW, NB = L::NVAR - NW;
-  constexpr bool MIXED = sizeof(T) == sizeof(float);
-  if (k >= ghost_count<D>(g)) return;
-  int c[3], s[3];
-  ghost_coords<D>(g, k, c);
-  s[0] = c[0];
-  s[1] = c[1];
-  s[2] = c[2];
-  unsigned neg = 0;
-  for (int limit = D - 1; limit >= 0;) {
-    int q = limit, L0 = -1;
-    for (; q >= 0; --q) {
-      bool covers = s[q] < 2 || s[q] > g.n[q] - 3;
-      if (!covers && g.btype[q] == BC_FIXED)
-        for (int e = 0; e < q; ++e)
-          if (s[e] == 0 || s[e] == g.n[e] - 1) covers = true;
-      if (covers) {
-        L0 = q;
-        break;
-      }
-    }
-    if (L0 < 0) break;                      // an inner cell: the source
-    if (g.btype[L0] == BC_FIXED) return;    // keeps its loaded value
-    neg ^= bc_neg(g, L0);
-    s[L0] = bc_source(g.btype[L0], D, g.n[L0], s[L0]);
-    limit = L0 - 1;
-  }
-  const long long j = gidx<D>(g, c), src = gidx<D>(g, s);
-  T ov[NW];
-  if (!MIXED) {
-#pragma unroll
-    for (int f = 0; f < NW; ++f) {
-      double v = a.out[fo32(f, g.N, src)];
-      if ((neg >> f) & 1u) v = -v;
-      a.out[fo32(f, g.N, j)] = v;
-      ov[f] = v;
-    }
-  } else if (a.kind == 4) {
-#pragma unroll
-    for (int f = 0; f < NW; ++f) {
-      float v = a.w32[fo32(f, g.N, src)], w = a.c32[fo32(f, g.N, src)];
-      if ((neg >> f) & 1u) {
-        v = -v;
-        w = -w;
-      }
-      a.w32[fo32(f, g.N, j)] = v;
-      a.c32[fo32(f, g.N, j)] = w;
-      ov[f] = v;
-    }
-  } else {
-#pragma unroll
-    for (int f = 0; f < NW; ++f) {
-      float v = a.out32[fo32(f, g.N, src)];
-      if ((neg >> f) & 1u) v = -v;
-      a.out32[fo32(f, g.N, j)] = v;
-      ov[f] = v;
-    }
-  }
-  double bgv[NB];
-#pragma unroll
-  for (int b = 0; b < NB; ++b)
-    bgv[b] = (b == L::RHOB - NW || p.has_bgb) ? __ldg(a.bg + fo32(b, g.N, j)) : 0.0;
-  if constexpr (MIXED)
-    reduce_cell_mixed<D>(g, p, ov, bgv, j, red);
-  else
-    reduce_cell<D>(g, p, ov, bgv, j, red);
-}
-
 // One RK stage on the tile (bx, by, bz) of one simulation; every thread of
 // the block calls it (it synchronises the block).  sm: tile_smem_elems<D, S>()
-// elements of T.
+// elements of T.  (Single-step runs, and 3-D runs without the workspace of
+// smaug_pass3.cuh.)
 template <int D, typename T, typename S>
 __device__ __forceinline__ void tile_body(const StageArgs &a, const Geo &g, const Phys &p, int bx, int by, int bz,
                                           T *sm, T *red) {
@@ -556,12 +584,12 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, const Geo &g, cons
   const double h = a.hslot > 0 ? a.sc->hst[a.hslot] : dt / a.hdiv;
   T cm[3] = {0, 0, 0};
 #pragma unroll
-  for (int d = 0; d < D; ++d) cm[d] = (T)red_get(a.sc->red[a.red_in], d);
+  for (int d = 0; d < D; ++d) cm[d] = num<T>(red_get(a.sc->red[a.red_in], d));
   int tile_ext[3] = {TX, TY, D == 3 ? TZ : 1};
   T idx1[3] = {0, 0, 0};
   if (active) {
 #pragma unroll
-    for (int d = 0; d < D; ++d) idx1[d] = (T)__ldg(g.rdx1[d] + c[d]);
+    for (int d = 0; d < D; ++d) idx1[d] = num<T>(__ldg(g.rdx1[d] + c[d]));
   }
   T dL[NW];
 #pragma unroll
@@ -610,11 +638,11 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, const Geo &g, cons
 
   // ------------------------------------------------ gravity
   if (active && p.has_grav) {
-    const T rho = C.v(L::RHO, idx), irt = (T)__drcp_rn((double)rho + C.vd(L::RHOB, idx));
+    const T rho = C.v(L::RHO, idx), irt = num<T>(__drcp_rn(dbl(rho) + C.vd(L::RHOB, idx)));
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-      dL[L::M0 + k] += (T)p.g[k] * rho;
-      dL[L::EN] += rho * (T)p.g[k] * C.v(L::M0 + k, idx) * irt;
+      dL[L::M0 + k] += num<T>(p.g[k]) * rho;
+      dL[L::EN] += rho * num<T>(p.g[k]) * C.v(L::M0 + k, idx) * irt;
     }
   }
   if constexpr (D == 2) {
@@ -724,7 +752,7 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, const Geo &g, cons
       const int r0 = qb.index(cc);
       const int fr = fb.index(cc);  // the cell's right face along d; its left face is fr - fs
       const int fs = d == 0 ? 1 : d == 1 ? fb.ext[0] : fb.ext[0] * fb.ext[1];
-      const T dxd = (T)__ldg(g.dx1[d] + c[d]);
+      const T dxd = num<T>(__ldg(g.dx1[d] + c[d]));
       // nu_R, nu_L of slot k at the cell shifted by `off` faces across d: dx
       // c_max c_hyp times the face ratios (0 off the inner cells, as the
       // reference's viscosity arrays are)
@@ -734,7 +762,7 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, const Geo &g, cons
           const int ff = k - (2 + D);
           fid = L::B0 + (ff >= d ? ff + 1 : ff);
         }
-        const T kk = dxd * cm[d] * (T)p.chyp[fid];
+        const T kk = dxd * cm[d] * num<T>(p.chyp[fid]);
         nr = in ? kk * V[k * nf + fr + off] : T(0);
         nl = in ? kk * V[k * nf + fr - fs + off] : T(0);
       };
@@ -745,7 +773,7 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, const Geo &g, cons
         double bb2 = 0;
 #pragma unroll
         for (int k = 0; k < D; ++k) bb2 += C.vd(L::BB0 + k, idx) * C.vd(L::BB0 + k, idx);
-        const T ptb = (T)((p.gamma - 1) * C.vd(L::EB, idx) - 0.5 * (p.gamma - 2) * bb2);
+        const T ptb = num<T>((p.gamma - 1) * C.vd(L::EB, idx) - 0.5 * (p.gamma - 2) * bb2);
         const bool z4d = z4(g, c, d);
 #pragma unroll
         for (int dir = 0; dir < D; ++dir) {
@@ -864,7 +892,8 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, const Geo &g, cons
     if constexpr (D == 3) dim_pass(std::integral_constant<int, 2>{});
   }
 
-  stage_epilogue<D, T>(a, g, p, C, c, active, idx, h, dL, numax, red);
+  if (numax > red[5] || numax != numax) red[5] = numax;
+  if (active) advance_cell_any<D, T>(a, g, p, c, idx, h, dL, red);
 }
 
 // One launch = one RK stage of one simulation, one block per tile.
@@ -873,18 +902,7 @@ __global__ void __launch_bounds__(256, 2) tile_stage_kernel(StageArgs a, Geo g, 
   extern __shared__ __align__(16) unsigned char smraw[];
   T red[6] = {0, 0, 0, 0, 0, 0};
   tile_body<D, T, TileShape<D>>(a, g, p, blockIdx.x, blockIdx.y, blockIdx.z, reinterpret_cast<T *>(smraw), red);
-  block_max_flush<6>(red, &a.sc->red[a.red_out]);
-}
-
-// The ghost pass after a tile_stage_kernel launch (grid-stride over the ghosts).
-template <int D, typename T>
-__global__ void __launch_bounds__(256) ghost_stage_kernel(StageArgs a, Geo g, Phys p) {
-  T red[6] = {0, 0, 0, 0, 0, 0};
-  const long long ng = ghost_count<D>(g);
-  const long long step = (long long)gridDim.x * blockDim.x;
-  for (long long k0 = (long long)blockIdx.x * blockDim.x; k0 < ng; k0 += step)
-    ghost_cell<D, T>(a, g, p, k0 + threadIdx.x, red);
-  block_max_flush<6>(red, &a.sc->red[a.red_out]);
+  block_max_flush<0, 6>(red, &a.sc->red[a.red_out]);
 }
 
 // shared memory elements (of the stencil type) the tile body needs

@@ -15,8 +15,8 @@
 //   phase C  per cell: the fluxes at the four neighbours along each
 //            dimension from their q slots and their 4th-order divergence,
 //            gravity, background energy terms, hyperdiffusion with
-//            nu = dx c_max c_hyp * ratio on the cell's faces, then the shared
-//            epilogue.
+//            nu = dx c_max c_hyp * ratio on the cell's faces; the sources go
+//            to the advance pass (advance_cell).
 // A q cell outside the grid along one dimension takes that dimension's pad
 // (0 on the right, q(5) on the left, as the reference's padded copies do);
 // the corners outside both are never read.
@@ -62,22 +62,22 @@ template <typename T>
 __device__ __forceinline__ void q_from(const QRaw<T> &r, double gam, T *q) {
   const T rho = r.rho, m0 = r.m0, m1 = r.m1, b0 = r.b0, b1 = r.b1, e = r.e, bb0 = r.bb0, bb1 = r.bb1;
   const double rhob = r.rhob;
-  const double irtd = __drcp_rn((double)rho + rhob);
-  const T irt = (T)irtd;
-  const double b2 = (double)b0 * (double)b0 + (double)b1 * (double)b1;
-  const double m2 = (double)m0 * (double)m0 + (double)m1 * (double)m1;
-  const double bbb = (double)b0 * (double)bb0 + (double)b1 * (double)bb1;
+  const double irtd = __drcp_rn(dbl(rho) + rhob);
+  const T irt = num<T>(irtd);
+  const double b2 = dbl(b0) * dbl(b0) + dbl(b1) * dbl(b1);
+  const double m2 = dbl(m0) * dbl(m0) + dbl(m1) * dbl(m1);
+  const double bbb = dbl(b0) * dbl(bb0) + dbl(b1) * dbl(bb1);
   q[0] = rho;
-  q[1] = (T)((double)e - 0.5 * (b2 + m2 * irtd));
+  q[1] = num<T>(dbl(e) - 0.5 * (b2 + m2 * irtd));
   q[2] = m0 * irt;
   q[3] = m1 * irt;
   q[4] = b0;
   q[5] = b1;
-  q[6] = rho + (T)rhob;
+  q[6] = rho + num<T>(rhob);
   q[7] = m0;
   q[8] = m1;
   q[9] = e;
-  q[10] = (T)((gam - 1.0) * ((double)e - 0.5 * m2 * irtd) - (gam - 2.0) * (bbb + 0.5 * b2));
+  q[10] = num<T>((gam - 1.0) * (dbl(e) - 0.5 * m2 * irtd) - (gam - 2.0) * (bbb + 0.5 * b2));
   q[11] = bb0;
   q[12] = bb1;
   q[13] = r.eb;
@@ -160,53 +160,6 @@ struct Box2 {
   static constexpr int ELEMS = OV1 + 5 * V1N;
 };
 
-// The rows of the tile that the epilogue reads are prefetched toward L2 at the start
-// of the tile, so that their DRAM latency overlaps phases A-C. Those rows are the
-// cell's RK base, the accumulator and the compensation where the stage reads them,
-// rho_b and the energy backgrounds, and the last dim's metric. Each (array, row)
-// segment of TX cells gets a prefetch at its first and its last byte. Every address
-// lies in its array: the rows are inner rows, and a row's TX cells from ox run at
-// most into the next row.
-template <typename T, int TX, int TY, int NT>
-__device__ __forceinline__ void prefetch_epilogue_rows(const StageArgs &a, const Geo &g, const Phys &p, int ox,
-                                                       int oy) {
-  using L = Lay<2>;
-  constexpr int NW = L::NW;
-  constexpr bool MIXED = sizeof(T) == sizeof(float);
-  const int nrow = min(TY, g.n[1] - 2 - oy);
-  const bool acc = MIXED ? a.kind >= 2 : (a.kind == 3 || a.kind == 4);
-  const bool comp = MIXED && a.kind == 4;
-  // arrays: base 0..NW-1, accumulator NW..2NW-1, compensation 2NW..3NW-1,
-  // backgrounds 3NW..3NW+3 (rho_b always), the last dim's metric 3NW+4
-  constexpr int NA = 3 * NW + 5;
-  for (int s = threadIdx.x; s < NA * TY; s += NT) {
-    const int arr = s / TY, row = s % TY;
-    if (row >= nrow) continue;
-    const unsigned cell = (unsigned)(ox + (oy + row) * g.st[1]);
-    const char *ptr = nullptr;
-    int es = (int)sizeof(T);
-    if (arr < NW) {
-      ptr = MIXED ? (const char *)(a.w32 + fo32(arr, g.N, cell)) : (const char *)(a.base + fo32(arr, g.N, cell));
-    } else if (arr < 2 * NW) {
-      if (acc)
-        ptr = MIXED ? (const char *)(a.acc32 + fo32(arr - NW, g.N, cell))
-                    : (const char *)(a.acc + fo32(arr - NW, g.N, cell));
-    } else if (arr < 3 * NW) {
-      if (comp) ptr = (const char *)(a.c32 + fo32(arr - 2 * NW, g.N, cell));
-    } else if (arr < 3 * NW + 4) {
-      const int b = arr - 3 * NW;
-      if (b == L::RHOB - NW || p.has_bgb) ptr = (const char *)(a.bg + fo32(b, g.N, cell));
-      es = 8;
-    } else {
-      ptr = (const char *)(g.dxlast + cell);
-      es = 8;
-    }
-    if (!ptr) continue;
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr));
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr + TX * es - 1));
-  }
-}
-
 // The q box of tile (nbx, nby) of the same simulation (the block's next work
 // item), prefetched toward L2: the stage input's fields and the backgrounds that
 // q_load reads, one prefetch per line of each row segment of the box, clamped to
@@ -244,7 +197,7 @@ __device__ __forceinline__ void prefetch_qbox_rows(const StageArgs &a, const Geo
 
 template <typename T, typename S>
 __device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, const Phys &p, int bx, int by, int nbx,
-                                           int nby, T *sm, T *red) {
+                                           int nby, T *sm, T &red) {
   using L = Lay<2>;
   using B = Box2<S>;
   constexpr int TX = S::TX, TY = S::TY, NT = TX * TY;
@@ -264,9 +217,7 @@ __device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, con
   const bool active = c[0] <= n0 - 3 && c[1] <= n1 - 3;
   const long long idx = active ? c[0] + (long long)c[1] * g.st[1] : 0;
   const CellT<2, T> C{MIXED ? (const T *)(const void *)a.in32 : (const T *)(const void *)a.in, a.bg, g.N};
-  const double h = a.hslot > 0 ? a.sc->hst[a.hslot] : a.sc->dt / a.hdiv;
-  const T cm[2] = {(T)red_get(a.sc->red[a.red_in], 0), (T)red_get(a.sc->red[a.red_in], 1)};
-  prefetch_epilogue_rows<T, TX, TY, NT>(a, g, p, ox, oy);
+  const T cm[2] = {num<T>(red_get(a.sc->red[a.red_in], 0)), num<T>(red_get(a.sc->red[a.red_in], 1))};
   if (nbx >= 0) prefetch_qbox_rows<T, TX, TY, NT>(a, g, p, nbx, nby);
 
   // ------------------------------------------------ phase A: q on the tile +-3
@@ -370,7 +321,7 @@ __device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, con
   T numax = 0;
   if (active) {
     const int tx = c[0] - ox, ty = c[1] - oy;
-    const T idx1[2] = {(T)__ldg(g.rdx1[0] + c[0]), (T)__ldg(g.rdx1[1] + c[1])};
+    const T idx1[2] = {num<T>(__ldg(g.rdx1[0] + c[0])), num<T>(__ldg(g.rdx1[1] + c[1]))};
     const int r0 = (tx + 3) + B::QX * (ty + 3);
     // flux divergences: -(8 (F_+1 - F_-1) - (F_+2 - F_-2)) / (12 dx), the
     // fluxes of the neighbours (inside the grid: the cell is an inner cell)
@@ -410,11 +361,11 @@ __device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, con
     div_terms(std::integral_constant<int, 1>{});
     // gravity
     if (p.has_grav) {
-      const T rho = C.v(L::RHO, idx), irt = (T)__drcp_rn((double)rho + C.vd(L::RHOB, idx));
+      const T rho = C.v(L::RHO, idx), irt = num<T>(__drcp_rn(dbl(rho) + C.vd(L::RHOB, idx)));
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        dL[L::M0 + k] += (T)p.g[k] * rho;
-        dL[L::EN] += rho * (T)p.g[k] * C.v(L::M0 + k, idx) * irt;
+        dL[L::M0 + k] += num<T>(p.g[k]) * rho;
+        dL[L::EN] += rho * num<T>(p.g[k]) * C.v(L::M0 + k, idx) * irt;
       }
     }
     if (p.divb) divb_sources<T>(C, g, p, c, idx, dL);
@@ -428,7 +379,7 @@ __device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, con
       if (p.has_bgb) {  // background energy terms along d (addenergyterms_cd2)
         const double bb0 = C.vd(L::BB0, idx), bb1 = C.vd(L::BB0 + 1, idx);
         const double bb2 = bb0 * bb0 + bb1 * bb1;
-        const T ptb = (T)((p.gamma - 1) * C.vd(L::EB, idx) - 0.5 * (p.gamma - 2) * bb2);
+        const T ptb = num<T>((p.gamma - 1) * C.vd(L::EB, idx) - 0.5 * (p.gamma - 2) * bb2);
         const bool z4d = z4(g, c, d);
 #pragma unroll
         for (int dir = 0; dir < 2; ++dir) {
@@ -449,14 +400,14 @@ __device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, con
       const int fo = 1 - d;                                  // the other dimension
       const int sv = d == 0 ? B::V0X : 1;                    // face stride along fo
       const int sq = fo == 0 ? 1 : B::QX;                    // q stride along fo
-      const T dxd = (T)__ldg(g.dx1[d] + c[d]);
+      const T dxd = num<T>(__ldg(g.dx1[d] + c[d]));
       // dx c_max c_hyp of each slot, and whether the neighbours along fo are
       // inner cells (the cell itself is: tiles cover inner cells only)
       T kk[5];
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
         const int fid = k == 0 ? L::RHO : k == 1 ? L::EN : k < 4 ? L::M0 + (k - 2) : L::B0 + (d == 0 ? 1 : 0);
-        kk[k] = dxd * cm[d] * (T)p.chyp[fid];
+        kk[k] = dxd * cm[d] * num<T>(p.chyp[fid]);
       }
       const int cfo = c[fo], nfo = fo == 0 ? n0 : n1;
       const bool inm = cfo - 1 >= 2, inp = cfo + 1 <= nfo - 3;
@@ -554,7 +505,8 @@ __device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, con
       dim_terms(std::integral_constant<int, 1>{});
     }
   }
-  stage_epilogue<2, T>(a, g, p, C, c, active, idx, h, dL, numax, red);
+  if (active) store_sources<2>(a, g, idx, dL);
+  if (numax > red || numax != numax) red = numax;
 }
 
 // Shared memory (elements of the stencil type) of a stage body: the
