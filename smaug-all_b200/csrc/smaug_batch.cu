@@ -2,13 +2,13 @@
 // include/smaug_b200.h).
 //
 // A batch holds many independent simulations of one ndim and one precision,
-// of any sizes, in one device arena.  A batch step is six launches for all
+// of any sizes, in one device arena.  A batch step is a few launches for all
 // of them together:
-//   batch_dt_kernel        per simulation: the reference's dt rule, and
+//   batch_turn_kernel      per simulation: the end of the step before (running
+//                          maxima, status), the reference's dt rule, and
 //                          whether it takes this step (steps left, status)
-//   batch stage kernel x4  one persistent launch per RK stage over the work
-//                          list of (simulation, tile) items
-//   batch_finish_kernel    per simulation: running maxima, status
+//   stage kernel(s) x4     one launch per RK stage in 2-D, three passes in 3-D
+//   advance kernel x4      the RK combination, ghosts and wave speeds
 // and a chunk of steps is replayed from a CUDA graph.  Simulations are added
 // and removed between steps (admission by arena footprint); finished ones
 // stop taking steps on the device without a host round trip.
@@ -28,12 +28,19 @@ namespace {
 
 constexpr int kGraphSteps = 16;  // steps per replay of the long graph
 
-__global__ void batch_dt_kernel(BatchInst *tab, long long *left, int *status, int n, int D) {
+// Per simulation, between steps: the end of the step it took (finish), and the
+// dt and the decision to take the next one (start).
+__global__ void batch_turn_kernel(BatchInst *tab, long long *left, int *status, int n, int D, int finish, int start) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   BatchInst &I = tab[i];
   if (!I.active) return;
   DevScalars *sc = I.sc;
+  if (finish && sc->go) {
+    finish_update(sc, 4);
+    status[i] = sc->status;
+  }
+  if (!start) return;
   if (left[i] > 0 && sc->status == 0) {
     dt_update(sc, I.phys, D);
     sc->go = 1;
@@ -42,15 +49,6 @@ __global__ void batch_dt_kernel(BatchInst *tab, long long *left, int *status, in
     sc->go = 0;
   }
   status[i] = sc->status;
-}
-
-__global__ void batch_finish_kernel(BatchInst *tab, int *status, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  BatchInst &I = tab[i];
-  if (!I.active || !I.sc->go) return;
-  finish_update(I.sc, 4);
-  status[i] = I.sc->status;
 }
 
 // Every simulation in the batch takes stage 1 (autotuning only: stage 1
@@ -326,8 +324,9 @@ void launch_rk_stage(smaug_batch *b, int k, cudaStream_t s) {
     smaug_batchk::launch_pass3(b->mixed, b->variant, b->d_tab, b->d_slabs, b->d_work, b->plan3, k, b->grid, s);
 }
 int launches_per_rk_stage(const smaug_batch *b) { return b->D == 2 ? 1 : 3 * (int)b->plan3.groups.size(); }
-// A step: dt, four stages each followed by its advance pass, finish.
-int launches_per_step(const smaug_batch *b) { return 6 + 4 * launches_per_rk_stage(b); }
+// n steps: dt, four stages each followed by its advance pass, finish, with
+// finish and the next step's dt in one launch.
+long long launches_of(const smaug_batch *b, int n) { return 1 + (5 + 4 * (long long)launches_per_rk_stage(b)) * n; }
 
 // The step stream waits for the admissions queued on the upload stream.
 int join_uploads(smaug_batch *b) {
@@ -371,9 +370,12 @@ int reclaim(smaug_batch *b, bool wait) {
   return SMAUG_OK;
 }
 
-void enqueue_step(smaug_batch *b, cudaStream_t s, bool timed = false) {
-  const int nb = (b->max_inst + 127) / 128;
-  batch_dt_kernel<<<nb, 128, 0, s>>>(b->d_tab, b->d_left, b->d_status, b->max_inst, b->D);
+void enqueue_turn(smaug_batch *b, cudaStream_t s, bool finish, bool start) {
+  batch_turn_kernel<<<(b->max_inst + 127) / 128, 128, 0, s>>>(b->d_tab, b->d_left, b->d_status, b->max_inst, b->D, finish,
+                                                              start);
+}
+
+void enqueue_stages(smaug_batch *b, cudaStream_t s, bool timed) {
   for (int k = 1; k <= 4; ++k) {
     cudaEvent_t e1 = nullptr;
     if (timed) {
@@ -392,13 +394,20 @@ void enqueue_step(smaug_batch *b, cudaStream_t s, bool timed = false) {
     smaug_batchk::launch_batch_advance(b->D, b->mixed, b->d_tab, b->d_awork, b->nawork, k, b->sms, s);
     if (e1) cudaEventRecord(e1, s);
   }
-  batch_finish_kernel<<<nb, 128, 0, s>>>(b->d_tab, b->d_status, b->max_inst);
+}
+
+void enqueue_steps(smaug_batch *b, cudaStream_t s, int n, bool timed = false) {
+  for (int i = 0; i < n; ++i) {
+    enqueue_turn(b, s, i > 0, true);
+    enqueue_stages(b, s, timed);
+  }
+  enqueue_turn(b, s, true, false);
 }
 
 int capture(smaug_batch *b, int steps, cudaGraphExec_t *out) {
   cudaGraph_t g = nullptr;
   BK(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal));
-  for (int i = 0; i < steps; ++i) enqueue_step(b, b->cap);
+  enqueue_steps(b, b->cap, steps);
   BK(cudaStreamEndCapture(b->cap, &g));
   cudaError_t e = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
@@ -690,8 +699,10 @@ int smaug_batch_step(smaug_batch *b, int nsteps) {
   }
   if (b->nwork == 0) return SMAUG_OK;
   if (b->profile) {
-    for (int i = 0; i < nsteps; ++i) enqueue_step(b, b->stream, true);
-    b->launches += (long long)launches_per_step(b) * nsteps;
+    if (nsteps > 0) {
+      enqueue_steps(b, b->stream, nsteps, true);
+      b->launches += launches_of(b, nsteps);
+    }
     BK(cudaGetLastError());
     return SMAUG_OK;
   }
@@ -705,11 +716,11 @@ int smaug_batch_step(smaug_batch *b, int nsteps) {
   }
   for (int i = 0; i + kGraphSteps <= nsteps; i += kGraphSteps) {
     BK(cudaGraphLaunch(b->gk, b->stream));
-    b->launches += (long long)launches_per_step(b) * kGraphSteps;
+    b->launches += launches_of(b, kGraphSteps);
   }
   for (int i = 0; i < nsteps % kGraphSteps; ++i) {
     BK(cudaGraphLaunch(b->g1, b->stream));
-    b->launches += launches_per_step(b);
+    b->launches += launches_of(b, 1);
   }
   return SMAUG_OK;
 }

@@ -57,7 +57,7 @@ struct Run : SimPlan {
   // (their kernel arguments hold the buffers and the physics; dropped when
   // those change)
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
-  long long graph_launches = 0;  // kernel launches per step in the graphs
+  long long graph_launches[2] = {0, 0};  // kernel launches of each graph
 };
 
 constexpr int kGraphSteps = 16;
@@ -79,6 +79,15 @@ __global__ void dt_kernel(DevScalars *sc, Phys p, int D) {
 
 __global__ void finish_kernel(DevScalars *sc, int last) {
   if (threadIdx.x == 0 && blockIdx.x == 0) finish_update(sc, last);
+}
+
+// The end of one step and the start of the next, one launch instead of two.
+__global__ void turn_kernel(DevScalars *sc, Phys p, int D, int last) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) {
+    finish_update(sc, last);
+    dt_update(sc, p, D);
+    sc->go = 1;
+  }
 }
 
 __global__ void reset_scalars_kernel(DevScalars *sc, double dt0) {
@@ -228,9 +237,11 @@ cudaError_t run_combine(Run &r) {
 inline int stages_per_step(const Run &r) { return r.rk4 ? 4 : 1; }
 
 // Enqueue stage k (1..stages_per_step) of a step: stage 1 opens the step with
-// the dt kernel, the last stage closes it with the finish kernel.
-cudaError_t run_stage(Run &r, int k) {
-  if (k == 1) {
+// the dt kernel, the last stage closes it with the finish kernel; inside a run
+// of steps (first: nothing was stepped before in it, last: no step follows) one
+// kernel does both.
+cudaError_t run_stage(Run &r, int k, bool first = true, bool last = true) {
+  if (k == 1 && first) {
     dt_kernel<<<1, 1, 0, r.stream>>>(r.sc, r.phys, r.D);
     r.launches++;
   }
@@ -263,7 +274,10 @@ cudaError_t run_stage(Run &r, int k) {
     launch_stage(r, a);
   }
   if (k == stages_per_step(r)) {
-    finish_kernel<<<1, 1, 0, r.stream>>>(r.sc, k);
+    if (last)
+      finish_kernel<<<1, 1, 0, r.stream>>>(r.sc, k);
+    else
+      turn_kernel<<<1, 1, 0, r.stream>>>(r.sc, r.phys, r.D, k);
     r.launches++;
   }
   return cudaGetLastError();
@@ -274,7 +288,7 @@ cudaError_t run_steps(Run &r, int nsteps) {
   const int ns = stages_per_step(r);
   for (int it = 0; it < nsteps; ++it)
     for (int k = 1; k <= ns; ++k) {
-      const cudaError_t e = run_stage(r, k);
+      const cudaError_t e = run_stage(r, k, it == 0, it == nsteps - 1);
       if (e != cudaSuccess) return e;
     }
   return cudaSuccess;
@@ -488,7 +502,7 @@ cudaError_t ensure_graphs(Run &r) {
     const long long l0 = r.launches;
     e = run_steps(r, len[k]);
     const cudaError_t e2 = cudaStreamEndCapture(r.stream, &g);
-    r.graph_launches = (r.launches - l0) / len[k];
+    r.graph_launches[k] = r.launches - l0;
     r.launches = l0;
     if (e != cudaSuccess) return e;
     if (e2 != cudaSuccess) return e2;
@@ -505,12 +519,12 @@ cudaError_t run_steps_graphed(Run &r, int nsteps) {
   for (; nsteps >= kGraphSteps; nsteps -= kGraphSteps) {
     const cudaError_t e = cudaGraphLaunch(r.graph[0], r.stream);
     if (e != cudaSuccess) return e;
-    r.launches += r.graph_launches * kGraphSteps;
+    r.launches += r.graph_launches[0];
   }
   for (; nsteps > 0; --nsteps) {
     const cudaError_t e = cudaGraphLaunch(r.graph[1], r.stream);
     if (e != cudaSuccess) return e;
-    r.launches += r.graph_launches;
+    r.launches += r.graph_launches[1];
   }
   return cudaSuccess;
 }

@@ -104,6 +104,25 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long *slot, doub
   atomicMax(slot, (unsigned long long)__double_as_longlong(v));
 }
 
+// Reads of a simulation's scalars by the kernels of a stage, past L1: with
+// dependent launches (below) a line of them may have been cached by the kernel
+// before, while others' atomics updated it in L2.
+__device__ __forceinline__ double sc_red(const DevScalars *sc, int slot, int i) {
+  return __longlong_as_double((long long)__ldcg(&sc->red[slot].v[i]));
+}
+__device__ __forceinline__ int sc_go(const DevScalars *sc) { return __ldcg(&sc->go); }
+__device__ __forceinline__ double sc_h(const DevScalars *sc, int slot) { return __ldcg(&sc->hst[slot]); }
+
+// Programmatic dependent launch: the kernels of a stage are launched while the
+// one before runs, wait for its end here (its writes are visible then) and let
+// the next one launch.  Launched only after the wait, a kernel never starts
+// before the one two ahead of it has ended; none of them reads through L1 what
+// it, or the kernel before it, writes.
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __host__ __device__ __forceinline__ double red_get(const Reduce &r, int i) {
   double x;
   memcpy(&x, &r.v[i], sizeof(double));

@@ -156,10 +156,11 @@ __device__ __forceinline__ int images(const Geo &g, int d, int x, int *xs, unsig
 }
 
 // cfast/courant maxima of the state `o` written at cell idx (with that cell's
-// background values).
+// background values); returns the speed along the last dim.
 template <int D>
-__device__ __forceinline__ void reduce_cell(const Geo &g, const Phys &p, const double *o, const double *bgv,
-                                            long long idx, double *r) {
+__device__ __forceinline__ double reduce_cell(const Geo &g, const Phys &p, const double *o, const double *bgv,
+                                              long long idx, double *r) {
+  double last = 0;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     double cf = cfast_vals<D>(o, bgv, d, p.gamma);
@@ -168,8 +169,10 @@ __device__ __forceinline__ void reduce_cell(const Geo &g, const Phys &p, const d
       double cour = cf / (__ldg(g.dxlast + idx));
       if (cour > r[3] || cour != cour) r[3] = cour;
       if (idx >= g.K && (cour > r[4] || cour != cour)) r[4] = cour;
+      last = cf;
     }
   }
+  return last;
 }
 
 template <int D>

@@ -216,9 +216,11 @@ __device__ __forceinline__ void q_all(const CellT<D, T> &c, long long i, int d, 
 // maxima come out the same bits either way.
 __device__ __forceinline__ float sqrt_approx(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
 
+// Returns the correctly rounded speed of the last dim, or -1 if the cell was
+// done after the fast pass.
 template <int D>
-__device__ __forceinline__ void reduce_cell_mixed(const Geo &g, const Phys &p, const float *o, const double *b,
-                                                  long long idx, float *r) {
+__device__ __forceinline__ float reduce_cell_mixed(const Geo &g, const Phys &p, const float *o, const double *b,
+                                                   long long idx, float *r) {
   using L = Lay<D>;
   const float irt = __frcp_rn(num<float>(dbl(o[L::RHO]) + b[1]));
   float m2 = 0.0f, b2 = 0.0f, bbb = 0.0f, bb2 = 0.0f;
@@ -257,8 +259,9 @@ __device__ __forceinline__ void reduce_cell_mixed(const Geo &g, const Phys &p, c
         if (idx >= g.K) need |= !(cour < r[4] * kBelow);
       }
     }
-    if (!need) return;
+    if (!need) return -1.0f;
   }
+  float last = 0.0f;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     const float bd = num<float>(b[2 + d] + dbl(o[L::B0 + d]));
@@ -270,8 +273,10 @@ __device__ __forceinline__ void reduce_cell_mixed(const Geo &g, const Phys &p, c
       const float cour = __fmul_rn(cff, __frcp_rn(num<float>(__ldg(g.dxlast + idx))));
       if (cour > r[3] || cour != cour) r[3] = cour;
       if (idx >= g.K && (cour > r[4] || cour != cour)) r[4] = cour;
+      last = cff;
     }
   }
+  return last;
 }
 
 // reduce_cell (FP64) behind a screen, as in reduce_cell_mixed: the speeds with
@@ -292,9 +297,11 @@ __device__ __forceinline__ double rcp_approx(double x) {
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
   return r;
 }
+// Returns the exact speed of the last dim, or -1 if the cell was done after the
+// screen.
 template <int D>
-__device__ __forceinline__ void reduce_cell_screened(const Geo &g, const Phys &p, const double *o, const double *b,
-                                                     long long idx, double *r) {
+__device__ __forceinline__ double reduce_cell_screened(const Geo &g, const Phys &p, const double *o, const double *b,
+                                                       long long idx, double *r) {
   using L = Lay<D>;
   const double irt = __drcp_rn(o[L::RHO] + b[1]);
   double m2 = 0, b2 = 0, bbb = 0, bb2 = 0;
@@ -324,7 +331,20 @@ __device__ __forceinline__ void reduce_cell_screened(const Geo &g, const Phys &p
       if (idx >= g.K) need |= !(cour < r[4] * kBelow);
     }
   }
-  if (need) reduce_cell<D>(g, p, o, b, idx, r);
+  return need ? reduce_cell<D>(g, p, o, b, idx, r) : -1.0;
+}
+
+// The courant number of a cell of speed cff at cell j, taken into the maxima,
+// with the operations of the two reductions.
+__device__ __forceinline__ void courant_at(const Geo &g, float cff, long long j, float *r) {
+  const float cour = __fmul_rn(cff, __frcp_rn(num<float>(__ldg(g.dxlast + j))));
+  if (cour > r[3] || cour != cour) r[3] = cour;
+  if (j >= g.K && (cour > r[4] || cour != cour)) r[4] = cour;
+}
+__device__ __forceinline__ void courant_at(const Geo &g, double cff, long long j, double *r) {
+  const double cour = cff / __ldg(g.dxlast + j);
+  if (cour > r[3] || cour != cour) r[3] = cour;
+  if (j >= g.K && (cour > r[4] || cour != cour)) r[4] = cour;
 }
 
 // Loads and stores of the advance pass: every value is touched once, so it
@@ -353,9 +373,10 @@ __device__ __forceinline__ void load_sources(const StageArgs &a, const Geo &g, l
 // Wave-speed maxima of the state v (of the inner cell or one of its images)
 // at cell j, with that cell's backgrounds (e_b and B_b are zero everywhere
 // without an energy background: only rho_b is read then).
+// Returns the speed of the last dim as the functions above.
 template <int D, typename T>
-__device__ __forceinline__ void reduce_at(const StageArgs &a, const Geo &g, const Phys &p, const T *v, long long j,
-                                          T *red) {
+__device__ __forceinline__ T reduce_at(const StageArgs &a, const Geo &g, const Phys &p, const T *v, long long j,
+                                       T *red) {
   using L = Lay<D>;
   constexpr int NW = L::NW, NB = L::NVAR - NW;
   double bgv[NB];
@@ -363,9 +384,9 @@ __device__ __forceinline__ void reduce_at(const StageArgs &a, const Geo &g, cons
   for (int b = 0; b < NB; ++b)
     bgv[b] = (b == L::RHOB - NW || p.has_bgb) ? __ldg(a.bg + fo32(b, g.N, j)) : 0.0;
   if constexpr (sizeof(T) == sizeof(float))
-    reduce_cell_mixed<D>(g, p, v, bgv, j, red);
+    return reduce_cell_mixed<D>(g, p, v, bgv, j, red);
   else
-    reduce_cell_screened<D>(g, p, v, bgv, j, red);
+    return reduce_cell_screened<D>(g, p, v, bgv, j, red);
 }
 
 // The end of a stage for one inner cell: the stage output base + h dL with the
@@ -484,6 +505,7 @@ __device__ __forceinline__ void advance_cell(const StageArgs &a, const Geo &g, c
   const int count = n0 * n1 * n2;
   long long j = idx;
   unsigned neg = 0;
+  T cff = 0;  // the cell's own speed along the last dim, if it was formed exactly
 #pragma unroll 1
   for (int k = 0;;) {
     T v[NW];
@@ -496,7 +518,17 @@ __device__ __forceinline__ void advance_cell(const StageArgs &a, const Geo &g, c
       stq(w + q, v[f]);
       if (MIXED && KIND == 4) stq(a.c32 + q, m ? -(float)lo[f] : (float)lo[f]);
     }
-    reduce_at<D, T>(a, g, p, v, j, red);  // what the next stage reads
+    // What the next stage reads.  An image without negated fields over the
+    // cell's own background has the cell's speeds: only its courant number,
+    // over the metric there, can differ (and the exact pass again, once per
+    // image, would be most of a small grid's advance).
+    if (k > 0 && neg == 0 && cff > T(0) && !p.has_bgb &&
+        __ldg(a.bg + fo32(L::RHOB - NW, g.N, j)) == __ldg(a.bg + fo32(L::RHOB - NW, g.N, idx))) {
+      courant_at(g, cff, j, red);
+    } else {
+      const T c0 = reduce_at<D, T>(a, g, p, v, j, red);
+      if (k == 0) cff = c0;
+    }
     if (++k >= count) break;
     const int i0 = k % n0, r = k / n0, i1 = r % n1, i2 = r / n1;
     j = (i0 == 0 ? c[0] : i0 == 1 ? xa : xb) + (i1 == 0 ? c[1] : i1 == 1 ? ya : yb) * g.st[1] +

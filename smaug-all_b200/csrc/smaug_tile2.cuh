@@ -196,8 +196,8 @@ __device__ __forceinline__ void prefetch_qbox_rows(const StageArgs &a, const Geo
 }
 
 template <typename T, typename S>
-__device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, const Phys &p, int bx, int by, int nbx,
-                                           int nby, T *sm, T &red) {
+__device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, const Phys &p, const T *scm, int bx, int by,
+                                           int nbx, int nby, T *sm, T &red) {
   using L = Lay<2>;
   using B = Box2<S>;
   constexpr int TX = S::TX, TY = S::TY, NT = TX * TY;
@@ -217,7 +217,7 @@ __device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, con
   const bool active = c[0] <= n0 - 3 && c[1] <= n1 - 3;
   const long long idx = active ? c[0] + (long long)c[1] * g.st[1] : 0;
   const CellT<2, T> C{MIXED ? (const T *)(const void *)a.in32 : (const T *)(const void *)a.in, a.bg, g.N};
-  const T cm[2] = {num<T>(red_get(a.sc->red[a.red_in], 0)), num<T>(red_get(a.sc->red[a.red_in], 1))};
+  const T cm[2] = {scm[0], scm[1]};  // c_max of the stage input
   if (nbx >= 0) prefetch_qbox_rows<T, TX, TY, NT>(a, g, p, nbx, nby);
 
   // ------------------------------------------------ phase A: q on the tile +-3
