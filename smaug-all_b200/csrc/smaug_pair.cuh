@@ -53,4 +53,60 @@ __device__ __forceinline__ f2 pfma(f2 a, f2 b, f2 c) {
 }
 __device__ __forceinline__ f2 pneg(f2 a) { return a * f2_splat(-1.0f); }
 
+// One lane with the same operations, as instructions the compiler leaves alone
+// too, so that each is rounded as a lane of f2 rounds it.
+struct f1 {
+  float r;
+};
+__device__ __forceinline__ f1 operator+(f1 a, f1 b) {
+  f1 o;
+  asm("add.rn.ftz.f32 %0, %1, %2;" : "=f"(o.r) : "f"(a.r), "f"(b.r));
+  return o;
+}
+__device__ __forceinline__ f1 operator-(f1 a, f1 b) {
+  f1 o;
+  asm("sub.rn.ftz.f32 %0, %1, %2;" : "=f"(o.r) : "f"(a.r), "f"(b.r));
+  return o;
+}
+__device__ __forceinline__ f1 operator*(f1 a, f1 b) {
+  f1 o;
+  asm("mul.rn.ftz.f32 %0, %1, %2;" : "=f"(o.r) : "f"(a.r), "f"(b.r));
+  return o;
+}
+__device__ __forceinline__ f1 pfma(f1 a, f1 b, f1 c) {
+  f1 o;
+  asm("fma.rn.ftz.f32 %0, %1, %2, %3;" : "=f"(o.r) : "f"(a.r), "f"(b.r), "f"(c.r));
+  return o;
+}
+__device__ __forceinline__ f1 pneg(f1 a) { return {-a.r}; }
+
+// Common names of both: all lanes alike, a value per lane (f1 takes the
+// first), a lane, and zero in the lanes whose flag is off.
+template <typename P>
+__device__ __forceinline__ P splat(float a);
+template <>
+__device__ __forceinline__ f1 splat<f1>(float a) {
+  return {a};
+}
+template <>
+__device__ __forceinline__ f2 splat<f2>(float a) {
+  return f2_splat(a);
+}
+template <typename P>
+__device__ __forceinline__ P pack(float lo, float hi);
+template <>
+__device__ __forceinline__ f1 pack<f1>(float lo, float) {
+  return {lo};
+}
+template <>
+__device__ __forceinline__ f2 pack<f2>(float lo, float hi) {
+  return f2_make(lo, hi);
+}
+__device__ __forceinline__ float lane(f1 x, int) { return x.r; }
+__device__ __forceinline__ float lane(f2 x, int k) { return k ? f2_hi(x) : f2_lo(x); }
+template <typename P>
+__device__ __forceinline__ P keep(bool lo, bool hi, P x) {
+  return pack<P>(lo ? lane(x, 0) : 0.0f, hi ? lane(x, 1) : 0.0f);
+}
+
 }  // namespace SMAUG_NS
