@@ -271,23 +271,29 @@ int rebuild(smaug_batch *b) {
     int t[3];
     batch_tile_shape(3, b->variant, t);
     b->plan3.build(sims, t, b->mixed);
+    if (b->plan3.bytes > b->work3_bytes) {  // queued steps use the workspace
+      BK(cudaStreamSynchronize(b->stream));
+      cudaFree(b->work3);
+      b->work3 = nullptr;
+      b->work3_bytes = 0;
+      cudaError_t e = cudaErrorMemoryAllocation;
+      for (size_t limit = kSlabBytes; e == cudaErrorMemoryAllocation && limit >= (size_t)4 << 20; limit /= 4) {
+        (void)cudaGetLastError();  // a failed attempt
+        if (limit != kSlabBytes) b->plan3.build(sims, t, b->mixed, limit);
+        e = cudaMalloc(&b->work3, b->plan3.bytes);
+      }
+      BK(e);
+      b->work3_bytes = b->plan3.bytes;
+    }
     w.swap(b->plan3.items);
   }
   const size_t nslab = b->plan3.slabs.size();
   int rc = SMAUG_OK;
-  if (gw.size() > b->awork_cap || w.size() > b->work_cap || nslab > b->slabs_cap ||
-      b->plan3.bytes > b->work3_bytes) {  // queued steps read the device lists and use the workspace
+  if (gw.size() > b->awork_cap || w.size() > b->work_cap || nslab > b->slabs_cap) {  // queued steps read the lists
     BK(cudaStreamSynchronize(b->stream));
     if ((rc = list_grow(b, &b->d_awork, &b->awork_cap, gw.size())) != SMAUG_OK) return rc;
     if ((rc = list_grow(b, &b->d_work, &b->work_cap, w.size())) != SMAUG_OK) return rc;
     if ((rc = list_grow(b, &b->d_slabs, &b->slabs_cap, nslab)) != SMAUG_OK) return rc;
-    if (b->plan3.bytes > b->work3_bytes) {
-      cudaFree(b->work3);
-      b->work3 = nullptr;
-      b->work3_bytes = 0;
-      BK(cudaMalloc(&b->work3, b->plan3.bytes));
-      b->work3_bytes = b->plan3.bytes;
-    }
   }
   b->plan3.place(b->work3);
   const int k = b->st_cur;

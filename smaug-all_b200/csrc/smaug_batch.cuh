@@ -66,8 +66,9 @@ struct Plan3 {
   std::vector<Group> groups;
   size_t bytes = 0;  // workspace
 
-  // sims: (slot, geometry) of every simulation; t: the terms tile.
-  void build(const std::vector<std::pair<int, Geo>> &sims, const int *t, bool mixed) {
+  // sims: (slot, geometry) of every simulation; t: the terms tile; limit: of
+  // the workspace (the caller halves it where the device has less to give).
+  void build(const std::vector<std::pair<int, Geo>> &sims, const int *t, bool mixed, size_t limit = kSlabBytes) {
     slabs.clear();
     items.clear();
     groups.clear();
@@ -99,7 +100,7 @@ struct Plan3 {
       const int inner = g.n[2] - 4;
       const size_t plane = (size_t)g.st[2] * es * (kDerived3 + kFaces3);
       // equal slabs of at least 4 planes, each within the target where it can be
-      const int most = std::max(4, (int)(kSlabBytes / plane) - 4);
+      const int most = std::max(4, (int)(limit / plane) - 4);
       const int cuts = std::max(1, std::min((inner + most - 1) / most, inner / 4));
       for (int k = 0; k < cuts; ++k) {
         Slab3 s{};
@@ -111,7 +112,7 @@ struct Plan3 {
         s.NP = (int)(((s.pz1 - s.pz0) * g.st[2] + 7) & ~7LL);
         s.NV = (int)(((s.z1 - s.z0 + 2) * g.st[2] + 7) & ~7LL);
         const size_t pb = align((size_t)s.NP * kDerived3 * es), vb = align((size_t)s.NV * kFaces3 * es);
-        if (used + pb + vb > kSlabBytes) flush();
+        if (used + pb + vb > limit) flush();
         s.P = (void *)used;
         s.V = (void *)(used + pb);
         used += pb + vb;

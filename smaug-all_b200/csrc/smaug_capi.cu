@@ -5,9 +5,12 @@
 //   dt_kernel                 the reference's moddton dt block
 //                             (iosmaug.cpp:855-898), from maxima that the
 //                             previous stage already reduced on the device
-//   stage kernel x 4 (or 1)   fused RK stages (fluxes + hyperdiffusion +
-//                             ghost fill + wave-speed maxima)
-//   finish_kernel             running maxviscoef, carry the maxima
+//   stage kernel x 4 (or 1)   RK stages (fluxes + hyperdiffusion; three passes
+//                             in 3-D), each followed by the advance kernel (RK
+//                             combination, ghost fill, wave-speed maxima); the
+//                             single step does all of it in one kernel
+//   finish_kernel             running maxviscoef, carry the maxima (inside a run
+//                             of steps one kernel with the next dt)
 // No host round trip happens inside a step (the reference copies struct
 // params and often the whole derived-field array between host and device
 // dozens of times per step).
@@ -174,8 +177,12 @@ cudaError_t run_plan3(Run &r) {
   if (r.D != 3 || !r.rk4 || r.exact) return cudaSuccess;
   int t[3];
   batch_tile_shape(3, batch_default_variant(3, r.mixed), t);
-  r.plan3.build({{0, r.geo}}, t, r.mixed);
-  cudaError_t e = cudaMalloc(&r.work3, r.plan3.bytes);
+  cudaError_t e = cudaErrorMemoryAllocation;
+  for (size_t limit = kSlabBytes; e == cudaErrorMemoryAllocation && limit >= (size_t)4 << 20; limit /= 4) {
+    (void)cudaGetLastError();  // a failed attempt
+    r.plan3.build({{0, r.geo}}, t, r.mixed, limit);
+    e = cudaMalloc(&r.work3, r.plan3.bytes);
+  }
   if (e == cudaSuccess) e = cudaMalloc(&r.slabs, sizeof(Slab3) * r.plan3.slabs.size());
   if (e == cudaSuccess) e = cudaMalloc(&r.items, sizeof(WorkItem) * r.plan3.items.size());
   if (e != cudaSuccess) return e;

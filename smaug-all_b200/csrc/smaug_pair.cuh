@@ -3,8 +3,11 @@
 //
 // Each lane is rounded exactly as the scalar instruction of the same name
 // rounds it (round to nearest even, subnormals flushed as the -ftz=true build
-// flushes them), so a computation written with these operations gives the
-// same bits as its scalar form.  Negation is a multiply by -1 (exact, and it
+// flushes them).  A product that goes into a sum is to be written with pfma:
+// ptxas contracts a packed mul and the add behind it into one fma where it sees
+// fit (measured: C - A * B and C + A * B differ from their scalar forms in one
+// value of five), which it does not do to the scalar .rn forms.  Written so, a
+// computation gives the same bits on one lane (f1) and on two.  Negation is a multiply by -1 (exact, and it
 // keeps the sign of zero), since the packed fma has no negated operand form.
 #pragma once
 
