@@ -256,9 +256,10 @@ int smaug_step_noalloc(const smaug_params *prm, const double *delx_dev, const do
  * simulation).  A batch holds many independent simulations of one ndim and
  * one precision, each of its own size and parameters, in one device arena
  * allocated at creation.  smaug_batch_step advances every simulation that
- * still has steps left by one RK4 step per step: one launch per RK stage for
- * all of them (a persistent kernel over a (simulation, tile) work list),
- * replayed from CUDA graphs.  Each simulation keeps its own dt (the
+ * still has steps left by one RK4 step per step: the same few launches per RK
+ * stage for all of them (persistent kernels over work lists), replayed from
+ * CUDA graphs.  (A 3-D batch takes a stage workspace beside the arena, up to
+ * 512 MB, at its first step; a 3-D rk4 context at its creation.)  Each simulation keeps its own dt (the
  * reference's rule, or fixed), maxima and status; its results are the same
  * as those of a context with the same smaug_params (the same kernel
  * arithmetic).  Simulations are added and removed between calls, on the
