@@ -232,7 +232,7 @@ int stage_grow(smaug_batch *b, E **buf, size_t *cap, size_t need) {
   if (need <= *cap) return SMAUG_OK;
   if (*buf) cudaFreeHost(*buf);
   *buf = nullptr;
-  *cap = std::max(need, (size_t)1024) * 2;
+  *cap = std::max(need, (size_t)4096) * 4;  // (a few hundred KB: growing waits for the queued steps)
   BK(cudaMallocHost((void **)buf, sizeof(E) * *cap));
   return SMAUG_OK;
 }
@@ -243,7 +243,7 @@ int list_grow(smaug_batch *b, E **list, size_t *cap, size_t need) {
   if (need <= *cap) return SMAUG_OK;
   cudaFree(*list);
   *list = nullptr;
-  *cap = std::max(need, (size_t)1024) * 2;
+  *cap = std::max(need, (size_t)4096) * 4;  // (a few hundred KB: growing waits for the queued steps)
   BK(cudaMalloc(list, sizeof(E) * *cap));
   return SMAUG_OK;
 }
@@ -255,6 +255,7 @@ int list_grow(smaug_batch *b, E **list, size_t *cap, size_t need) {
 int rebuild(smaug_batch *b) {
   std::vector<WorkItem> w, gw;
   std::vector<std::pair<int, Geo>> sims;
+  long long chunks = 0;
   for (int i = 0; i < b->max_inst; ++i) {
     if (!b->slots[i].used) continue;
     set_tiles(b, b->h_tab[i]);
@@ -264,8 +265,15 @@ int rebuild(smaug_batch *b) {
     else
       for (int y = 0; y < tl[1]; ++y)
         for (int x = 0; x < tl[0]; ++x) w.push_back({i, x, y, 0});
+    chunks += advance_items(b->h_tab[i].geo, b->D);
+  }
+  // advance items: a chunk each, or four where there are plenty for every
+  // block (a shorter list to build, copy and read)
+  const int per = chunks >= 64LL * b->sms ? 4 : 1;
+  for (int i = 0; i < b->max_inst; ++i) {
+    if (!b->slots[i].used) continue;
     const int na = advance_items(b->h_tab[i].geo, b->D);
-    for (int t = 0; t < na; ++t) gw.push_back({i, t, 0, 0});
+    for (int t = 0; t < na; t += per) gw.push_back({i, t, std::min(per, na - t), 0});
   }
   if (b->D == 3) {
     int t[3];

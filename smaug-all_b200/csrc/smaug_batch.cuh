@@ -24,8 +24,8 @@ struct BatchInst {
 // Work list entry: simulation slot and tile index within it.
 struct WorkItem {
   int inst;
-  int tile;    // stage items: the tile's x index; advance items: the chunk
-  int by, bz;  // stage items: the tile's y and z indices
+  int tile;    // stage items: the tile's x index; advance items: the first chunk
+  int by, bz;  // stage items: the tile's y and z indices; advance items: by chunks
 };
 
 // The 3-D stage runs over slabs: inner planes z0 .. z1-1 of one simulation with
