@@ -232,7 +232,7 @@ int stage_grow(smaug_batch *b, E **buf, size_t *cap, size_t need) {
   if (need <= *cap) return SMAUG_OK;
   if (*buf) cudaFreeHost(*buf);
   *buf = nullptr;
-  *cap = std::max(need, (size_t)4096) * 4;  // (a few hundred KB: growing waits for the queued steps)
+  *cap = std::max(need, (size_t)4096) * 2;
   BK(cudaMallocHost((void **)buf, sizeof(E) * *cap));
   return SMAUG_OK;
 }
@@ -243,7 +243,7 @@ int list_grow(smaug_batch *b, E **list, size_t *cap, size_t need) {
   if (need <= *cap) return SMAUG_OK;
   cudaFree(*list);
   *list = nullptr;
-  *cap = std::max(need, (size_t)4096) * 4;  // (a few hundred KB: growing waits for the queued steps)
+  *cap = std::max(need, (size_t)4096) * 2;
   BK(cudaMalloc(list, sizeof(E) * *cap));
   return SMAUG_OK;
 }
