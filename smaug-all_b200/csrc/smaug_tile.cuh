@@ -285,8 +285,11 @@ __device__ __forceinline__ float reduce_cell_mixed(const Geo &g, const Phys &p, 
 // a few roundings of cf^2, at most 1e-7 of cf after the root; the
 // approximations themselves 2^-20), so a cell that stays more than 1e-5 below
 // the running maxima cannot raise them.  Any other cell, a NaN included, takes
-// reduce_cell: the maxima keep their bits.  (Nine divisions and six square
-// roots in software per 3-D cell otherwise.)
+// reduce_cell: the maxima keep their bits.  So does a cell whose discriminant is
+// zero but for rounding (sound and Alfven speed along d agree): reduce_cell's
+// may be negative there and its speed NaN, which has to be seen whatever the
+// thread has seen before.  (Nine divisions and six square roots in software per
+// 3-D cell otherwise.)
 __device__ __forceinline__ double rsqrt_approx(double x) {
   double r;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
@@ -317,14 +320,20 @@ __device__ __forceinline__ double reduce_cell_screened(const Geo &g, const Phys 
   const double cf = (b2 + bb2 + 2.0 * bbb) * irt + cs2;
   constexpr double kBelow = 1.0 - 1e-5;
   const double rdx = rcp_approx(__ldg(g.dxlast + idx));
+  // How small the root of the discriminant |b_d^2 / rho_t - c_s^2| may be before
+  // rounding decides its sign: in either evaluation the discriminant carries a
+  // few roundings of cf^2 (its root 3e-8 of cf), and c_s^2 a few of the energies
+  // that p_k is recovered from (1e-13: 450 units of 2^-52).
+  const double low =
+      1e-6 * cf + 1e-13 * p.gamma * (fabs(o[L::EN]) + fabs(b[0]) + m2 * irt + b2 + bb2) * irt;
   bool need = false;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     const double bd = b[2 + d] + o[L::B0 + d];
     const double disc = cf * cf - 4.0 * cs2 * (bd * bd) * irt;
-    const double cfi = 0.5 * (cf + (disc > 0.0 ? disc * rsqrt_approx(disc) : disc));
+    const double cfi = 0.5 * (cf + disc * rsqrt_approx(disc));
     const double cff = cfi * rsqrt_approx(cfi) + fabs(o[L::M0 + d] * irt);
-    need |= !(cff < r[d] * kBelow);
+    need |= !(disc > low * low) || !(cff < r[d] * kBelow);
     if (d == D - 1) {
       const double cour = cff * rdx;
       need |= !(cour < r[3] * kBelow);
