@@ -104,23 +104,48 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long *slot, doub
   atomicMax(slot, (unsigned long long)__double_as_longlong(v));
 }
 
-// Reads of a simulation's scalars by the kernels of a stage, past L1: with
-// dependent launches (below) a line of them may have been cached by the kernel
-// before, while others' atomics updated it in L2.
-__device__ __forceinline__ double sc_red(const DevScalars *sc, int slot, int i) {
-  return __longlong_as_double((long long)__ldcg(&sc->red[slot].v[i]));
-}
-__device__ __forceinline__ int sc_go(const DevScalars *sc) { return __ldcg(&sc->go); }
-__device__ __forceinline__ double sc_h(const DevScalars *sc, int slot) { return __ldcg(&sc->hst[slot]); }
-
 // Programmatic dependent launch: the kernels of a stage are launched while the
 // one before runs, wait for its end here (its writes are visible then) and let
 // the next one launch.  Launched only after the wait, a kernel never starts
-// before the one two ahead of it has ended; none of them reads through L1 what
-// it, or the kernel before it, writes.
+// before the one two ahead of it has ended.  What a kernel before has written --
+// the state, the sources, the workspace, a simulation's scalars -- is read
+// behind the wait by ordinary loads (below): a non-coherent load (__ldg,
+// ld.global.nc) is for data that nothing writes while the kernel exists, the
+// backgrounds, the metric, the descriptors and the work lists.
 __device__ __forceinline__ void grid_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Loads of what the kernels before have written.  Volatile: the compiler keeps
+// them behind the wait.
+__device__ __forceinline__ float ldw(const float *p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ldw(const double *p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+
+// The same of a simulation's scalars, past L1: atomics of other blocks update
+// them in L2.
+__device__ __forceinline__ double sc_red(const DevScalars *sc, int slot, int i) {
+  double v;
+  asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(&sc->red[slot].v[i]));
+  return v;
+}
+__device__ __forceinline__ int sc_go(const DevScalars *sc) {
+  int v;
+  asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(&sc->go));
+  return v;
+}
+__device__ __forceinline__ double sc_h(const DevScalars *sc, int slot) {
+  double v;
+  asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(&sc->hst[slot]));
+  return v;
 }
 
 __host__ __device__ __forceinline__ double red_get(const Reduce &r, int i) {

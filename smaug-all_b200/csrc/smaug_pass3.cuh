@@ -48,17 +48,17 @@ struct alignas(16) Four {
 // there are.
 __device__ __forceinline__ Two<float> ldv(const Two<float> *p) {
   Two<float> v;
-  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
   return v;
 }
 __device__ __forceinline__ Two<double> ldv(const Two<double> *p) {
   Two<double> v;
-  asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
   return v;
 }
 __device__ __forceinline__ Four<float> ldv4(const Two<float> *p) {
   Four<float> v;
-  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ Four<double> ldv4(const Two<double> *p) {
@@ -98,36 +98,51 @@ struct Work3 {
 };
 
 // ---------------------------------------------------------------- derive
-// One thread per cell; bound by its loads and stores (36 B in and 56 B out per
-// cell in mixed precision).  The FP64 parts (p_T and the internal energy, both
-// recovered by cancellation) are formed here once per cell and stage.
+// kDeriveChunk / 256 cells per thread; bound by its loads and stores (36 B in and
+// 56 B out per cell in mixed precision).  The FP64 parts (p_T and the internal
+// energy, both recovered by cancellation) are formed here once per cell and
+// stage.  An ordinary load stays behind the stores before it, so where a block
+// has an SM to itself, the state of all four cells is loaded before the first
+// of them is stored (blast wave 26^3 mixed, us per launch: 10.3, so 8.5); where
+// other warps cover a load's latency, the registers of that cost more than it
+// gives (128^3 mixed 43.4 and 49.5, 85^3 FP64 24.4 and 28.0).
 template <typename T>
-__device__ __forceinline__ void derive_cell(const StageArgs &a, const Geo &g, const Phys &p, const Work3<T> &W,
+struct Raw3 {
+  T rho, e, m[3], b[3];
+};
+template <typename T>
+__device__ __forceinline__ void derive_load(const CellT<3, T> &C, int idx, Raw3<T> &r) {
+  using L = Lay<3>;
+  r.rho = C.v(L::RHO, idx);
+  r.e = C.v(L::EN, idx);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    r.m[k] = C.v(L::M0 + k, idx);
+    r.b[k] = C.v(L::B0 + k, idx);
+  }
+}
+template <typename T>
+__device__ __forceinline__ void derive_cell(const CellT<3, T> &C, const Phys &p, const Work3<T> &W, const Raw3<T> &r,
                                             int idx, int pi) {
   using L = Lay<3>;
-  constexpr bool MIXED = sizeof(T) == sizeof(float);
-  const CellT<3, T> C{MIXED ? (const T *)(const void *)a.in32 : (const T *)(const void *)a.in, a.bg, g.N};
-  const T rho = C.v(L::RHO, idx), e = C.v(L::EN, idx);
   const double rhob = C.vd(L::RHOB, idx);
-  const double irtd = __drcp_rn(dbl(rho) + rhob);
+  const double irtd = __drcp_rn(dbl(r.rho) + rhob);
   const T irt = num<T>(irtd);
-  T m[3], b[3], bb[3] = {0, 0, 0};
+  T bb[3] = {0, 0, 0};
   double b2 = 0, m2 = 0, bbb = 0;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    m[k] = C.v(L::M0 + k, idx);
-    b[k] = C.v(L::B0 + k, idx);
     if (p.has_bgb) bb[k] = C.v(L::BB0 + k, idx);
-    b2 += dbl(b[k]) * dbl(b[k]);
-    m2 += dbl(m[k]) * dbl(m[k]);
-    bbb += dbl(b[k]) * dbl(bb[k]);
+    b2 += dbl(r.b[k]) * dbl(r.b[k]);
+    m2 += dbl(r.m[k]) * dbl(r.m[k]);
+    bbb += dbl(r.b[k]) * dbl(bb[k]);
   }
-  const T ei = num<T>(dbl(e) - 0.5 * (b2 + m2 * irtd));
-  const T pt = num<T>((p.gamma - 1.0) * (dbl(e) - 0.5 * m2 * irtd) - (p.gamma - 2.0) * (bbb + 0.5 * b2));
+  const T ei = num<T>(dbl(r.e) - 0.5 * (b2 + m2 * irtd));
+  const T pt = num<T>((p.gamma - 1.0) * (dbl(r.e) - 0.5 * m2 * irtd) - (p.gamma - 2.0) * (bbb + 0.5 * b2));
 #pragma unroll
-  for (int k = 0; k < 3; ++k) stv(W.P + W.H(k, pi), b[k], m[k] * irt);
-  stv((Four<T> *)(W.P + W.MP(pi)), m[0], m[1], m[2], pt);
-  stv((Four<T> *)(W.P + W.R(pi)), rho + num<T>(rhob), e, rho, ei);
+  for (int k = 0; k < 3; ++k) stv(W.P + W.H(k, pi), r.b[k], r.m[k] * irt);
+  stv((Four<T> *)(W.P + W.MP(pi)), r.m[0], r.m[1], r.m[2], pt);
+  stv((Four<T> *)(W.P + W.R(pi)), r.rho + num<T>(rhob), r.e, r.rho, ei);
   if (p.has_bgb) stv((Four<T> *)(W.P + W.BG(pi)), bb[0], bb[1], bb[2], C.v(L::EB, idx));
 }
 
@@ -188,18 +203,10 @@ __device__ __forceinline__ void line_faces(const Work3<T> &W, int p0, int v0, in
     for (int m = 0; m < SEG; ++m, o += (unsigned)(2 * s))
       if (f0 + m <= f1) stv((Four<T> *)(W.V + o), a[m], b[m], c[m], e ? e[m] : T(0));
   };
+  // (rho, e_int) first: in this order the ratios that wait for a store are the
+  // fewest registers (72 -> 56 in mixed precision; blast wave 128^3 94.1 -> 87.1 us
+  // per launch)
   T r[4][SEG];
-  {
-    Two<T> q[SEG + 5];
-    load(W.H(f, 0), 1, q);
-    face_run2<T, SEG>(q, r[0], r[1]);
-  }
-  {
-    Two<T> q[SEG + 5];
-    load(W.H(h, 0), 1, q);
-    face_run2<T, SEG>(q, r[2], r[3]);
-  }
-  store(W.X(d, v0 + f0 * s), r[0], r[1], r[2], r[3]);
   {
     Two<T> q[SEG + 5];
     load(W.R(0) + 1, 2, q);  // (rho, e_int): the second half of R
@@ -211,6 +218,17 @@ __device__ __forceinline__ void line_faces(const Work3<T> &W, int p0, int v0, in
     face_run2<T, SEG>(q, r[3], r[2]);  // (b_d's ratio is not used)
   }
   store(W.Y(d, v0 + f0 * s), r[0], r[1], r[2], nullptr);
+  {
+    Two<T> q[SEG + 5];
+    load(W.H(f, 0), 1, q);
+    face_run2<T, SEG>(q, r[0], r[1]);
+  }
+  {
+    Two<T> q[SEG + 5];
+    load(W.H(h, 0), 1, q);
+    face_run2<T, SEG>(q, r[2], r[3]);
+  }
+  store(W.X(d, v0 + f0 * s), r[0], r[1], r[2], r[3]);
 }
 
 // ---------------------------------------------------------------- terms

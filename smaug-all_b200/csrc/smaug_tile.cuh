@@ -110,11 +110,11 @@ struct CellT {
   long long N;
   // field f at cell i in the stencil type
   __device__ __forceinline__ T v(int f, long long i) const {
-    return f < Lay<D>::NW ? __ldg(in + fo32(f, N, i)) : num<T>(__ldg(bg + fo32(f - Lay<D>::NW, N, i)));
+    return f < Lay<D>::NW ? ldw(in + fo32(f, N, i)) : num<T>(__ldg(bg + fo32(f - Lay<D>::NW, N, i)));
   }
   // field f at cell i in FP64
   __device__ __forceinline__ double vd(int f, long long i) const {
-    return f < Lay<D>::NW ? dbl(__ldg(in + fo32(f, N, i))) : __ldg(bg + fo32(f - Lay<D>::NW, N, i));
+    return f < Lay<D>::NW ? dbl(ldw(in + fo32(f, N, i))) : __ldg(bg + fo32(f - Lay<D>::NW, N, i));
   }
 };
 
