@@ -97,6 +97,15 @@ struct Pending {
   cudaEvent_t ev_main = nullptr, ev_io = nullptr;
 };
 
+// Memory that starts as a part of a larger allocation, grows into its own and
+// keeps what it outgrew (freeing waits for the GPU, and queued work may still
+// use it).
+struct Block {
+  char *p = nullptr;
+  size_t bytes = 0;
+  std::vector<char *> own;  // allocations of its own, the last one in use
+};
+
 constexpr int kSnaps = 4;  // poll snapshots in flight
 
 // Per slot: the steps it has left and its status (set at admission, on the
@@ -118,23 +127,26 @@ struct smaug_batch {
   char *arena = nullptr;
   size_t arena_bytes = 0;
   std::map<size_t, size_t> free_;  // offset -> size
+  char *d_base = nullptr, *h_base = nullptr;  // one allocation each: table, counters and lists; the pinned buffers
   BatchInst *d_tab = nullptr;
   long long *d_left = nullptr;
   int *d_status = nullptr;
   std::vector<BatchInst> h_tab;
   std::vector<Slot> slots;
+  // The work lists, one after another in one block on the device: advance
+  // chunks, stage items, slabs.  Its first room is what the arena's simulations
+  // need unless they are tiny; growing doubles, so that what was outgrown is
+  // together no larger than what is in use.
+  Block lists;
   WorkItem *d_work = nullptr;
-  WorkItem *d_awork = nullptr;  // advance chunks
-  size_t awork_cap = 0;
-  // 3-D: the plan of a stage over the current simulations, its slab list on
-  // the device (its items are d_work) and the workspace
-  Plan3 plan3;
+  WorkItem *d_awork = nullptr;
   Slab3 *d_slabs = nullptr;
-  size_t slabs_cap = 0;
+  // 3-D: the plan of a stage over the current simulations (its items are
+  // d_work) and the workspace
+  Plan3 plan3;
   char *work3 = nullptr;
   size_t work3_bytes = 0;
   int nawork = 0;
-  size_t work_cap = 0;
   int nwork = 0, grid = 0, variant = 0, sms = 148;
   bool dirty = true;
   cudaGraphExec_t g1 = nullptr, gk = nullptr;
@@ -162,10 +174,7 @@ struct smaug_batch {
   int last_snap = -1;  // ring entry of the last snapshot waited for (asynchronous reads follow it)
   // pinned staging of the work lists and the table (two sets, used in turn)
   BatchInst *st_tab[2] = {};
-  WorkItem *st_work[2] = {}, *st_awork[2] = {};
-  Slab3 *st_slabs[2] = {};
-  size_t st_slabs_cap[2] = {};
-  size_t st_work_cap[2] = {}, st_awork_cap[2] = {};
+  Block st_lists[2];
   cudaEvent_t st_ev[2] = {};
   int st_cur = 0;
 };
@@ -225,33 +234,32 @@ void set_tiles(const smaug_batch *b, BatchInst &I) {
   for (int d = 0; d < 3; ++d) I.tiles[d] = d < b->D ? (I.geo.n[d] - 4 + t[d] - 1) / t[d] : 1;
 }
 
-// Grow a pinned staging buffer (its copies from two rebuilds ago are done: the
-// caller waited for its event).
-template <typename E>
-int stage_grow(smaug_batch *b, E **buf, size_t *cap, size_t need) {
-  if (need <= *cap) return SMAUG_OK;
-  if (*buf) cudaFreeHost(*buf);
-  *buf = nullptr;
-  *cap = std::max(need, (size_t)4096) * 2;
-  BK(cudaMallocHost((void **)buf, sizeof(E) * *cap));
-  return SMAUG_OK;
+// Make room for `need` bytes.  An allocation while steps are queued can take
+// many ms (2 to 75 for lists of 640 KB behind a batch of 24, a fresh mapping
+// waiting for the GPU), hence the first room at creation.
+template <typename Alloc>
+cudaError_t block_grow(Block &k, size_t need, Alloc alloc) {
+  if (need <= k.bytes) return cudaSuccess;
+  char *p = nullptr;
+  const cudaError_t e = alloc((void **)&p, 2 * need);
+  if (e != cudaSuccess) return e;
+  k.own.push_back(p);
+  k.p = p;
+  k.bytes = 2 * need;
+  return cudaSuccess;
 }
 
-// Grow a device list (the caller waited for the steps that read it).
-template <typename E>
-int list_grow(smaug_batch *b, E **list, size_t *cap, size_t need) {
-  if (need <= *cap) return SMAUG_OK;
-  cudaFree(*list);
-  *list = nullptr;
-  *cap = std::max(need, (size_t)4096) * 2;
-  BK(cudaMalloc(list, sizeof(E) * *cap));
-  return SMAUG_OK;
+// Bytes the work lists start with: an item per 256 cells and kernel that walks
+// a list, for as many cells as the arena holds (208 B a cell or more; small grids
+// have more items to the cell and may grow the lists), to 4 MB.
+size_t first_lists(size_t arena_bytes) {
+  return align256(std::min(std::max(arena_bytes / 1024, (size_t)64 << 10), (size_t)4 << 20));
 }
 
 // Rebuild the work list and the persistent grid for the current simulations
 // and tile shape.  The table and the lists go to the device from pinned
 // staging buffers (two sets, used in turn), so nothing here waits for the
-// steps already queued, except when a device list must grow.
+// steps already queued, except a list that must grow.
 int rebuild(smaug_batch *b) {
   std::vector<WorkItem> w, gw;
   std::vector<std::pair<int, Geo>> sims;
@@ -296,30 +304,24 @@ int rebuild(smaug_batch *b) {
     w.swap(b->plan3.items);
   }
   const size_t nslab = b->plan3.slabs.size();
-  int rc = SMAUG_OK;
-  if (gw.size() > b->awork_cap || w.size() > b->work_cap || nslab > b->slabs_cap) {  // queued steps read the lists
-    BK(cudaStreamSynchronize(b->stream));
-    if ((rc = list_grow(b, &b->d_awork, &b->awork_cap, gw.size())) != SMAUG_OK) return rc;
-    if ((rc = list_grow(b, &b->d_work, &b->work_cap, w.size())) != SMAUG_OK) return rc;
-    if ((rc = list_grow(b, &b->d_slabs, &b->slabs_cap, nslab)) != SMAUG_OK) return rc;
-  }
   b->plan3.place(b->work3);
+  const size_t at_work = align256(sizeof(WorkItem) * gw.size()), at_slabs = at_work + align256(sizeof(WorkItem) * w.size());
+  const size_t bytes = at_slabs + sizeof(Slab3) * nslab;
   const int k = b->st_cur;
-  b->st_cur ^= 1;
   BK(cudaEventSynchronize(b->st_ev[k]));  // the copies out of set k, two rebuilds ago
-  if ((rc = stage_grow(b, &b->st_awork[k], &b->st_awork_cap[k], gw.size())) != SMAUG_OK) return rc;
-  if ((rc = stage_grow(b, &b->st_work[k], &b->st_work_cap[k], w.size())) != SMAUG_OK) return rc;
-  if ((rc = stage_grow(b, &b->st_slabs[k], &b->st_slabs_cap[k], nslab)) != SMAUG_OK) return rc;
+  BK(block_grow(b->st_lists[k], bytes, [](void **p, size_t n) { return cudaMallocHost(p, n); }));
+  BK(block_grow(b->lists, bytes, [](void **p, size_t n) { return cudaMalloc(p, n); }));
+  b->st_cur ^= 1;
+  b->d_awork = (WorkItem *)b->lists.p;
+  b->d_work = (WorkItem *)(b->lists.p + at_work);
+  b->d_slabs = (Slab3 *)(b->lists.p + at_slabs);
+  char *st = b->st_lists[k].p;
+  if (!gw.empty()) std::memcpy(st, gw.data(), sizeof(WorkItem) * gw.size());
+  if (!w.empty()) std::memcpy(st + at_work, w.data(), sizeof(WorkItem) * w.size());
+  if (nslab) std::memcpy(st + at_slabs, b->plan3.slabs.data(), sizeof(Slab3) * nslab);
   std::memcpy(b->st_tab[k], b->h_tab.data(), sizeof(BatchInst) * b->max_inst);
   BK(cudaMemcpyAsync(b->d_tab, b->st_tab[k], sizeof(BatchInst) * b->max_inst, cudaMemcpyHostToDevice, b->stream));
-  auto put = [&](auto *dev, auto *staging, const auto *src, size_t n) {
-    if (n == 0) return cudaSuccess;
-    std::memcpy(staging, src, sizeof(*src) * n);
-    return cudaMemcpyAsync(dev, staging, sizeof(*src) * n, cudaMemcpyHostToDevice, b->stream);
-  };
-  BK(put(b->d_awork, b->st_awork[k], gw.data(), gw.size()));
-  BK(put(b->d_work, b->st_work[k], w.data(), w.size()));
-  BK(put(b->d_slabs, b->st_slabs[k], b->plan3.slabs.data(), nslab));
+  if (bytes) BK(cudaMemcpyAsync(b->lists.p, st, bytes, cudaMemcpyHostToDevice, b->stream));
   BK(cudaEventRecord(b->st_ev[k], b->stream));
   b->nawork = (int)gw.size();
   b->nwork = (int)w.size();
@@ -468,22 +470,31 @@ int smaug_batch_create(int ndim, int precision, int device, size_t arena_bytes, 
   BK(cudaStreamCreateWithFlags(&b->up, cudaStreamNonBlocking));
   BK(cudaStreamCreateWithFlags(&b->io, cudaStreamNonBlocking));
   BK(cudaEventCreateWithFlags(&b->up_done, cudaEventDisableTiming));
-  for (int k = 0; k < kSnaps; ++k) {
-    BK(cudaMallocHost((void **)&b->snap_h[k], sizeof(long long) * max_sims));
-    BK(cudaEventCreateWithFlags(&b->snap_ev[k], cudaEventDisableTiming));
-  }
-  for (int k = 0; k < 2; ++k) {
-    BK(cudaMallocHost((void **)&b->st_tab[k], sizeof(BatchInst) * max_sims));
-    BK(cudaEventCreateWithFlags(&b->st_ev[k], cudaEventDisableTiming));
-  }
+  for (auto &ev : b->snap_ev) BK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  for (auto &ev : b->st_ev) BK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   BK(cudaMalloc(&b->arena, b->arena_bytes));
   b->free_[0] = b->arena_bytes;
-  BK(cudaMalloc(&b->d_tab, sizeof(BatchInst) * max_sims));
-  BK(cudaMalloc(&b->d_left, sizeof(long long) * max_sims));
-  BK(cudaMalloc(&b->d_status, sizeof(int) * max_sims));
-  BK(cudaMemsetAsync(b->d_tab, 0, sizeof(BatchInst) * max_sims, b->stream));
-  BK(cudaMemsetAsync(b->d_left, 0, sizeof(long long) * max_sims, b->stream));
-  BK(cudaMemsetAsync(b->d_status, 0, sizeof(int) * max_sims, b->stream));
+  const size_t tab = align256(sizeof(BatchInst) * max_sims), left = align256(sizeof(long long) * max_sims);
+  const size_t status = align256(sizeof(int) * max_sims), lists = first_lists(b->arena_bytes);
+  BK(cudaMallocHost((void **)&b->h_base, kSnaps * left + 2 * (tab + lists)));
+  char *h = b->h_base;
+  for (auto &snap : b->snap_h) {
+    snap = (long long *)h;
+    h += left;
+  }
+  for (int k = 0; k < 2; ++k) {
+    b->st_tab[k] = (BatchInst *)h;
+    b->st_lists[k].p = h + tab;
+    b->st_lists[k].bytes = lists;
+    h += tab + lists;
+  }
+  BK(cudaMalloc(&b->d_base, tab + left + status + lists));
+  b->d_tab = (BatchInst *)b->d_base;
+  b->d_left = (long long *)(b->d_base + tab);
+  b->d_status = (int *)(b->d_base + tab + left);
+  b->lists.p = b->d_base + tab + left + status;
+  b->lists.bytes = lists;
+  BK(cudaMemsetAsync(b->d_base, 0, tab + left + status, b->stream));
   BK(cudaStreamSynchronize(b->stream));
   return SMAUG_OK;
 }
@@ -497,29 +508,21 @@ int smaug_batch_destroy(smaug_batch *b) {
   drop_graphs(b);
   for (auto e : b->ev) cudaEventDestroy(e);
   cudaFree(b->arena);
-  cudaFree(b->d_tab);
-  cudaFree(b->d_left);
-  cudaFree(b->d_status);
-  cudaFree(b->d_work);
-  cudaFree(b->d_awork);
-  cudaFree(b->d_slabs);
+  cudaFree(b->d_base);
+  for (char *p : b->lists.own) cudaFree(p);
   cudaFree(b->work3);
   for (auto &q : b->pending) {
     if (q.ev_main) cudaEventDestroy(q.ev_main);
     if (q.ev_io) cudaEventDestroy(q.ev_io);
   }
   for (auto e : b->ev_pool) cudaEventDestroy(e);
-  for (int k = 0; k < kSnaps; ++k) {
-    if (b->snap_h[k]) cudaFreeHost(b->snap_h[k]);
-    if (b->snap_ev[k]) cudaEventDestroy(b->snap_ev[k]);
-  }
-  for (int k = 0; k < 2; ++k) {
-    if (b->st_tab[k]) cudaFreeHost(b->st_tab[k]);
-    if (b->st_work[k]) cudaFreeHost(b->st_work[k]);
-    if (b->st_awork[k]) cudaFreeHost(b->st_awork[k]);
-    if (b->st_slabs[k]) cudaFreeHost(b->st_slabs[k]);
-    if (b->st_ev[k]) cudaEventDestroy(b->st_ev[k]);
-  }
+  if (b->h_base) cudaFreeHost(b->h_base);
+  for (auto &st : b->st_lists)
+    for (char *p : st.own) cudaFreeHost(p);
+  for (auto ev : b->snap_ev)
+    if (ev) cudaEventDestroy(ev);
+  for (auto ev : b->st_ev)
+    if (ev) cudaEventDestroy(ev);
   if (b->up_done) cudaEventDestroy(b->up_done);
   if (b->stream) cudaStreamDestroy(b->stream);
   if (b->cap) cudaStreamDestroy(b->cap);
