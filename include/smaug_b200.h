@@ -258,8 +258,13 @@ int smaug_step_noalloc(const smaug_params *prm, const double *delx_dev, const do
  * allocated at creation.  smaug_batch_step advances every simulation that
  * still has steps left by one RK4 step per step: the same few launches per RK
  * stage for all of them (persistent kernels over work lists), replayed from
- * CUDA graphs.  (A 3-D batch takes a stage workspace beside the arena, up to
- * 512 MB, at its first step; a 3-D rk4 context at its creation.)  Each simulation keeps its own dt (the
+ * CUDA graphs.  A 3-D batch takes a stage workspace
+ * beside the arena at its first step, up to three quarters of the arena's size
+ * (1.5 times it in FP64) or 512 MB, whichever is less; a 3-D rk4 context takes
+ * 168 B (FP64 336 B) per cell and halo, up to 512 MB, at its creation.  Planes
+ * so large that four of them need more (1.3 KB, FP64 2.6 KB, per cell of a
+ * plane) take that; a device with less to give gets a smaller workspace and
+ * slower steps.  Each simulation keeps its own dt (the
  * reference's rule, or fixed), maxima and status; its results are the same
  * as those of a context with the same smaug_params (the same kernel
  * arithmetic).  Simulations are added and removed between calls, on the

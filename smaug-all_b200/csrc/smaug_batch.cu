@@ -144,8 +144,7 @@ struct smaug_batch {
   // 3-D: the plan of a stage over the current simulations (its items are
   // d_work) and the workspace
   Plan3 plan3;
-  char *work3 = nullptr;
-  size_t work3_bytes = 0;
+  Workspace3 work3;
   int nawork = 0;
   int nwork = 0, grid = 0, variant = 0, sms = 148;
   bool dirty = true;
@@ -286,25 +285,24 @@ int rebuild(smaug_batch *b) {
   if (b->D == 3) {
     int t[3];
     batch_tile_shape(3, b->variant, t);
-    b->plan3.build(sims, t, b->mixed);
-    if (b->plan3.bytes > b->work3_bytes) {  // queued steps use the workspace
-      BK(cudaStreamSynchronize(b->stream));
-      cudaFree(b->work3);
-      b->work3 = nullptr;
-      b->work3_bytes = 0;
-      cudaError_t e = cudaErrorMemoryAllocation;
-      for (size_t limit = kSlabBytes; e == cudaErrorMemoryAllocation && limit >= (size_t)4 << 20; limit /= 4) {
-        (void)cudaGetLastError();  // a failed attempt
-        if (limit != kSlabBytes) b->plan3.build(sims, t, b->mixed, limit);
-        e = cudaMalloc(&b->work3, b->plan3.bytes);
-      }
-      BK(e);
-      b->work3_bytes = b->plan3.bytes;
-    }
+    // (what simulations that fill the arena need, their halos included: 0.6 or 1.1
+    // bytes of workspace to one of theirs)
+    const size_t want = b->arena_bytes / 4 * (b->mixed ? 3 : 6);
+    BK(b->plan3.fit(
+        b->work3, sims, t, b->mixed, want,
+        [](void **p, size_t n) {
+          const cudaError_t e = cudaMalloc(p, n);
+          (void)cudaGetLastError();  // a refusal is handled
+          return e;
+        },
+        [b](char *p) {  // queued steps use it
+          cudaStreamSynchronize(b->stream);
+          cudaFree(p);
+        }));
     w.swap(b->plan3.items);
   }
   const size_t nslab = b->plan3.slabs.size();
-  b->plan3.place(b->work3);
+  b->plan3.place(b->work3.p);
   const size_t at_work = align256(sizeof(WorkItem) * gw.size()), at_slabs = at_work + align256(sizeof(WorkItem) * w.size());
   const size_t bytes = at_slabs + sizeof(Slab3) * nslab;
   const int k = b->st_cur;
@@ -510,7 +508,7 @@ int smaug_batch_destroy(smaug_batch *b) {
   cudaFree(b->arena);
   cudaFree(b->d_base);
   for (char *p : b->lists.own) cudaFree(p);
-  cudaFree(b->work3);
+  cudaFree(b->work3.p);
   for (auto &q : b->pending) {
     if (q.ev_main) cudaEventDestroy(q.ev_main);
     if (q.ev_io) cudaEventDestroy(q.ev_io);

@@ -48,11 +48,22 @@ constexpr int kDerived3 = 18, kFaces3 = 24;
 constexpr int kDeriveChunk = 1024, kFaceChunk = 512, kFaceSegs = 128;
 // Faces a thread takes along y and z.
 constexpr int face_seg(bool mixed) { return mixed ? 8 : 4; }
-// Workspace limit of one group of slabs (a slab has at least 4 planes).  Slabs
-// bound the memory; small ones that stay in L2 between their passes were
-// slower, each pass paying its ramp and tail (blast wave 128^3 mixed, ms per
-// step: 512 MB 1.86, 128 MB 2.09, 64 MB 2.33).
+// Workspace limit of one group of slabs.  Slabs bound the memory; small ones that
+// stay in L2 between their passes were slower, each pass paying its ramp and tail
+// (blast wave 128^3 mixed, ms per step: 512 MB 1.86, 128 MB 2.09, 64 MB 2.33).  A
+// slab has at least four planes, its halo being as large as they are, and takes
+// what they need (1.3 KB, in FP64 2.6 KB, per cell of a plane) where that is more;
+// only under a lower limit, where the device has less to give, do slabs go down to
+// one plane.
 constexpr size_t kSlabBytes = (size_t)512 << 20;
+constexpr size_t kLeastSlabBytes = (size_t)4 << 20;  // the last limit that is tried
+
+// The workspace of a context or a batch: kept from plan to plan, with the limit
+// that plans keep to (lowered for good where the memory for more was refused).
+struct Workspace3 {
+  char *p = nullptr;
+  size_t bytes = 0, limit = kSlabBytes;
+};
 
 // The work of one 3-D stage: groups of slabs that run one after another
 // through the same workspace, each with its items for the three passes
@@ -66,8 +77,52 @@ struct Plan3 {
   std::vector<Group> groups;
   size_t bytes = 0;  // workspace
 
+  // Plan for the simulations and find the workspace: the one in use if a plan
+  // within its limit fits it, else a larger one, first beside it, so that a refusal
+  // leaves it as it was and the plan is cut to it; at last, without it, smaller
+  // ones.  want: what to take rather than the bare need, so that later plans fit
+  // (at most the limit; twice the one in use in any case).  alloc(void **, bytes)
+  // returns a cudaError_t; release(p) waits for queued work that uses p and
+  // frees it.
+  template <typename Alloc, typename Release>
+  cudaError_t fit(Workspace3 &ws, const std::vector<std::pair<int, Geo>> &sims, const int *t, bool mixed, size_t want,
+                  Alloc alloc, Release release) {
+    build(sims, t, mixed, ws.limit);
+    if (bytes <= ws.bytes) return cudaSuccess;
+    cudaError_t e = cudaErrorMemoryAllocation;
+    auto refused = [&](size_t n) {
+      char *p = nullptr;
+      e = alloc((void **)&p, n);
+      if (e == cudaSuccess) {
+        if (ws.p) release(ws.p);
+        ws.p = p;
+        ws.bytes = n;
+      }
+      return e == cudaErrorMemoryAllocation;
+    };
+    const size_t room = std::max(bytes, std::min(ws.limit, std::max(want, 2 * ws.bytes)));
+    if (!refused(room) || (room > bytes && !refused(bytes))) return e;
+    if (ws.p) {
+      build(sims, t, mixed, ws.bytes);
+      if (bytes <= ws.bytes) {
+        ws.limit = ws.bytes;
+        return cudaSuccess;
+      }
+      release(ws.p);
+      ws.p = nullptr;
+      ws.bytes = 0;
+    }
+    for (size_t limit = ws.limit; limit >= kLeastSlabBytes; limit /= 4) {
+      build(sims, t, mixed, limit);
+      if (refused(bytes)) continue;
+      if (e == cudaSuccess) ws.limit = limit;
+      return e;
+    }
+    return e;
+  }
+
   // sims: (slot, geometry) of every simulation; t: the terms tile; limit: of
-  // the workspace (the caller halves it where the device has less to give).
+  // the workspace.
   void build(const std::vector<std::pair<int, Geo>> &sims, const int *t, bool mixed, size_t limit = kSlabBytes) {
     slabs.clear();
     items.clear();
@@ -99,9 +154,10 @@ struct Plan3 {
       const Geo &g = sim.second;
       const int inner = g.n[2] - 4;
       const size_t plane = (size_t)g.st[2] * es * (kDerived3 + kFaces3);
-      // equal slabs of at least 4 planes, each within the target where it can be
-      const int most = std::max(4, (int)(limit / plane) - 4);
-      const int cuts = std::max(1, std::min((inner + most - 1) / most, inner / 4));
+      // equal slabs of at least `least` planes, each within the limit where it can be
+      const int least = limit < kSlabBytes ? 1 : 4;
+      const int most = std::max(least, (int)(limit / plane) - 4);
+      const int cuts = std::max(1, std::min((inner + most - 1) / most, inner / least));
       for (int k = 0; k < cuts; ++k) {
         Slab3 s{};
         s.inst = sim.first;

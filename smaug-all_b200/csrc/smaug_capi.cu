@@ -48,7 +48,7 @@ struct Run : SimPlan {
   Plan3 plan3;  // 3-D: the slabs and items of a stage, their device lists and workspace
   Slab3 *slabs = nullptr;
   WorkItem *items = nullptr;
-  char *work3 = nullptr;
+  Workspace3 work3;
   int ntiles = 0, sms = 148;
   int grid = 0;  // persistent grid of the batch stage kernel (blocks), at most ntiles
   int cur = 0;
@@ -177,16 +177,18 @@ cudaError_t run_plan3(Run &r) {
   if (r.D != 3 || !r.rk4 || r.exact) return cudaSuccess;
   int t[3];
   batch_tile_shape(3, batch_default_variant(3, r.mixed), t);
-  cudaError_t e = cudaErrorMemoryAllocation;
-  for (size_t limit = kSlabBytes; e == cudaErrorMemoryAllocation && limit >= (size_t)4 << 20; limit /= 4) {
-    (void)cudaGetLastError();  // a failed attempt
-    r.plan3.build({{0, r.geo}}, t, r.mixed, limit);
-    e = cudaMalloc(&r.work3, r.plan3.bytes);
-  }
+  cudaError_t e = r.plan3.fit(
+      r.work3, {{0, r.geo}}, t, r.mixed, 0,
+      [](void **p, size_t n) {
+        const cudaError_t c = cudaMalloc(p, n);
+        (void)cudaGetLastError();  // a refusal is handled
+        return c;
+      },
+      [](char *p) { cudaFree(p); });
   if (e == cudaSuccess) e = cudaMalloc(&r.slabs, sizeof(Slab3) * r.plan3.slabs.size());
   if (e == cudaSuccess) e = cudaMalloc(&r.items, sizeof(WorkItem) * r.plan3.items.size());
   if (e != cudaSuccess) return e;
-  r.plan3.place(r.work3);
+  r.plan3.place(r.work3.p);
   e = cudaMemcpyAsync(r.slabs, r.plan3.slabs.data(), sizeof(Slab3) * r.plan3.slabs.size(), cudaMemcpyHostToDevice,
                       r.stream);
   if (e == cudaSuccess)
@@ -255,7 +257,7 @@ cudaError_t run_stage(Run &r, int k, bool first = true, bool last = true) {
   StageArgs a{};
   a.bg = r.bg;
   a.sc = r.sc;
-  if (r.mixed || (r.rk4 && !r.exact && (r.D == 2 || r.work3))) {
+  if (r.mixed || (r.rk4 && !r.exact && (r.D == 2 || r.work3.p))) {
     // production fourstep, FP64 or mixed (FP32 stage states: S1 = W + dt/2
     // L(W), S2 = W + dt/2 L(S1), S3 = W + dt L(S2), A = (S1 + 2 S2 + S3 -
     // 4 W)/3 accumulated stage by stage, W <- W + dt/6 L(S3) + A); the stage
@@ -393,7 +395,7 @@ int smaug_destroy(smaug_ctx *ctx) {
   cudaFree(ctx->dxlast);
   cudaFree(r.sc);
   cudaFree(r.inst);
-  cudaFree(r.work3);
+  cudaFree(r.work3.p);
   cudaFree(r.slabs);
   cudaFree(r.items);
   drop_graphs(r);

@@ -34,6 +34,10 @@ def test_growing_lists_do_not_wait_for_queued_steps(need_gpu):
     admit_into_running_batch(2, problems.orszag_tang(128), problems.orszag_tang(1536, ny=1400), 8000)
 
 
+def test_growing_workspace_does_not_wait_for_queued_steps(need_gpu):
+    admit_into_running_batch(3, problems.blast_wave(40, seed=1), problems.blast_wave(120, seed=2), 2500)
+
+
 def test_lists_of_many_tiny_simulations(need_gpu):
     """Simulations so small that their items outgrow the room that the lists
     start with, before and while steps are queued."""
