@@ -185,9 +185,11 @@ cudaError_t run_plan3(Run &r) {
         return c;
       },
       [](char *p) { cudaFree(p); });
-  if (e == cudaSuccess) e = cudaMalloc(&r.slabs, sizeof(Slab3) * r.plan3.slabs.size());
-  if (e == cudaSuccess) e = cudaMalloc(&r.items, sizeof(WorkItem) * r.plan3.items.size());
+  const size_t at_slabs = sizeof(WorkItem) * r.plan3.items.size();  // items, then slabs
+  static_assert(sizeof(WorkItem) % alignof(Slab3) == 0, "slabs follow the items");
+  if (e == cudaSuccess) e = cudaMalloc(&r.items, at_slabs + sizeof(Slab3) * r.plan3.slabs.size());
   if (e != cudaSuccess) return e;
+  r.slabs = (Slab3 *)((char *)r.items + at_slabs);
   r.plan3.place(r.work3.p);
   e = cudaMemcpyAsync(r.slabs, r.plan3.slabs.data(), sizeof(Slab3) * r.plan3.slabs.size(), cudaMemcpyHostToDevice,
                       r.stream);
@@ -396,7 +398,6 @@ int smaug_destroy(smaug_ctx *ctx) {
   cudaFree(r.sc);
   cudaFree(r.inst);
   cudaFree(r.work3.p);
-  cudaFree(r.slabs);
   cudaFree(r.items);
   drop_graphs(r);
   for (auto e : ctx->ev) cudaEventDestroy(e);
@@ -499,12 +500,16 @@ int smaug_get_state_device(smaug_ctx *ctx, double *w, size_t count) {
 }
 
 // The steps of the production RK4 path as graph replays: the launch sequence
-// of a step is the same every step (the batch stage kernel over this
-// simulation's one-entry table, its ghost pass, the dt and finish kernels).
-cudaError_t ensure_graphs(Run &r) {
+// of a step is the same every step (the batch stage kernels over this
+// simulation's one-entry table, the advance pass, the dt and finish kernels).
+// Captured are the graphs that nsteps steps launch: the long one holds 145
+// kernels (3-D: 273), a large part of a short first call (four steps of a new
+// vortex 64^2 mixed 640 us with it, 358 without; blast 26^3 1225 and 758).
+cudaError_t ensure_graphs(Run &r, int nsteps) {
   const int len[2] = {kGraphSteps, 1};
+  const bool used[2] = {nsteps >= kGraphSteps, nsteps % kGraphSteps != 0};
   for (int k = 0; k < 2; ++k) {
-    if (r.graph[k]) continue;
+    if (r.graph[k] || !used[k]) continue;
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(r.stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
@@ -523,7 +528,7 @@ cudaError_t ensure_graphs(Run &r) {
 }
 
 cudaError_t run_steps_graphed(Run &r, int nsteps) {
-  const cudaError_t eg = ensure_graphs(r);
+  const cudaError_t eg = ensure_graphs(r, nsteps);
   if (eg != cudaSuccess) return eg;
   for (; nsteps >= kGraphSteps; nsteps -= kGraphSteps) {
     const cudaError_t e = cudaGraphLaunch(r.graph[0], r.stream);
@@ -583,7 +588,7 @@ int smaug_step_on(smaug_ctx *ctx, int nsteps, void *stream) {
   if (ctx->next_stage != 1) return fail(ctx, SMAUG_ERR_STATE, "a step begun by smaug_stage is not finished");
   CK(cudaSetDevice(ctx->device));
   // the graphs are captured on the context's own stream, never the caller's
-  if (ctx->run.rk4 && !ctx->run.exact && !ctx->profile) CK(ensure_graphs(ctx->run));
+  if (ctx->run.rk4 && !ctx->run.exact && !ctx->profile) CK(ensure_graphs(ctx->run, nsteps));
   return on_stream(ctx, (cudaStream_t)stream, [&] { return step_impl(ctx, nsteps); });
 }
 
