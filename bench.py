@@ -69,8 +69,13 @@ def load_peaks():
     return 6650.0, "fallback"
 
 
+# What a timed RK stage of the headline batch launches (the stage times' events
+# bracket both kernels), and the key of its DRAM traffic in the ncu summary.
+STAGE_KERNELS = "batch_stage_kernel<2,float> + batch_advance_kernel<2,float>"
+
+
 def load_traffic():
-    """DRAM bytes per stage launch from the committed ncu summary, if any."""
+    """DRAM bytes per RK stage from the committed ncu summary, if any."""
     p = ROOT / "profiles" / "stage_kernel_traffic.json"
     if p.exists():
         try:
@@ -825,7 +830,7 @@ def main():
     achieved = alg / (head["avg_stage_ms"] / 1e3) / 1e9
     peak, peak_kind = load_peaks()
     tr = load_traffic()
-    kernel = "batch_stage_kernel<2,float>"
+    kernel = STAGE_KERNELS
     # DRAM bytes per inner cell from the committed ncu capture, times this
     # run's inner cells (traffic grows with the cells a launch processes)
     per_cell = tr.get(kernel, {}).get("dram_bytes_per_inner_cell") if tr else None

@@ -204,9 +204,10 @@ int smaug_sync(smaug_ctx *ctx);
 int smaug_get_scalars(smaug_ctx *ctx, double out[8]);
 
 /*
- * Stage timing: when enabled, CUDA events bracket every stage kernel launch;
- * smaug_stage_times waits, returns the summed device time (ms) and the number
- * of timed launches since the last call, and resets.  (The reference's only
+ * Stage timing: when enabled, CUDA events bracket every RK stage (its stage
+ * kernel or 3-D passes, and the advance pass); smaug_stage_times waits, returns
+ * the summed device time (ms) and the number of timed stages since the last
+ * call, and resets.  (The reference's only
  * timing is the per-step wall clock printf, iosmaug.cpp:1515-1517.)
  */
 int smaug_profile_stages(smaug_ctx *ctx, int enable);

@@ -226,7 +226,7 @@ class Engine:
         self._check(self.lib.smaug_profile_stages(self.h, int(enable)), "smaug_profile_stages")
 
     def stage_times(self):
-        """(total ms, launches) of the stage kernels timed since the last call."""
+        """(total ms, count) of the RK stages timed since the last call."""
         ms = _D()
         n = ctypes.c_longlong()
         self._check(self.lib.smaug_stage_times(self.h, ctypes.byref(ms), ctypes.byref(n)), "smaug_stage_times")

@@ -153,7 +153,7 @@ class Batch:
         self._check(self.lib.smaug_batch_profile_stages(self.h, int(enable)), "smaug_batch_profile_stages")
 
     def stage_times(self):
-        """(total ms, launches) of the stage kernels timed since the last call."""
+        """(total ms, count) of the RK stages timed since the last call."""
         ms = ctypes.c_double()
         n = ctypes.c_longlong()
         self._check(self.lib.smaug_batch_stage_times(self.h, ctypes.byref(ms), ctypes.byref(n)),
