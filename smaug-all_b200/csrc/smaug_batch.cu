@@ -897,6 +897,12 @@ int smaug_batch_tune(smaug_batch *b, int reps, int *variant_out, double *ms_out,
       if (ms_out && v < nms) ms_out[v] = -1.0;
       continue;
     }
+    // the same launches as an earlier variant's: its time, timed once
+    const int first = batch_first_alike(b->D, v);
+    if (first < v) {
+      if (ms_out && v < nms) ms_out[v] = ms_out[first];
+      continue;
+    }
     b->variant = v;
     int rc = rebuild(b);
     if (rc != SMAUG_OK) return rc;

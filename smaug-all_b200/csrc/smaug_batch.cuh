@@ -222,7 +222,9 @@ inline int advance_items(const Geo &g, int D) {
 
 // Tile shapes and, in 2-D, occupancy targets (resident blocks per SM the
 // register allocation is made for) the stage kernel is built for; the autotuner
-// picks one.
+// picks one.  In 3-D one terms kernel takes every shape: the ten variants are
+// five shapes (those of the tile kernels that the numbers were given to), and
+// min_blocks says nothing.
 constexpr int kBatchVariants2 = 11;
 constexpr int kBatchVariants3 = 10;
 struct BatchVariant {
@@ -276,6 +278,17 @@ __host__ __device__ inline void batch_tile_shape(int D, int v, int *t) {
   t[0] = b.t[0];
   t[1] = b.t[1];
   t[2] = b.t[2];
+}
+
+// The first variant that launches what variant v does.
+__host__ __device__ inline int batch_first_alike(int D, int v) {
+  if (D == 2) return v;
+  const BatchVariant b = batch_variant(3, v);
+  for (int u = 0; u < v; ++u) {
+    const BatchVariant a = batch_variant(3, u);
+    if (a.t[0] == b.t[0] && a.t[1] == b.t[1] && a.t[2] == b.t[2]) return u;
+  }
+  return v;
 }
 
 }  // namespace smaug
