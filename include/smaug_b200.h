@@ -246,6 +246,11 @@ int smaug_stage_times(smaug_ctx *ctx, double *ms_total, long long *count);
  * captured into a CUDA graph.  scalars_out (8 doubles, as smaug_get_scalars,
  * may be NULL) and err (may be NULL) are host buffers.  FP64 only: precision
  * must be SMAUG_PREC_FP64.
+ *
+ * The results are those of a context with the same parameters: bit for bit in
+ * 2-D and in single-step mode (rk4 = 0), where both run the same kernels; in
+ * 3-D with rk4 = 1 to rounding, since a context's passes need a workspace that
+ * this call does not have, and it runs one kernel per stage instead.
  */
 #define SMAUG_NOALLOC_SCRATCH_BYTES (32u << 20)
 int smaug_step_noalloc(const smaug_params *prm, const double *delx_dev, const double *w_in_dev,
