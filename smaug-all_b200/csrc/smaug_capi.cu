@@ -123,9 +123,9 @@ void timed_launch(Run &r, F launch) {
 void launch_stage(Run &r, const StageArgs &a) {
   timed_launch(r, [&] {
     if (r.exact)
-      smaug_exact::launch_stage(r.D, false, a, r.geo, r.phys, r.stream);
+      smaug_exact::launch_stage(r.D, a, r.geo, r.phys, r.stream);
     else
-      smaug_fast::launch_stage(r.D, r.mixed, a, r.geo, r.phys, r.stream);
+      smaug_fast::launch_stage(r.D, a, r.geo, r.phys, r.stream);
   });
 }
 

@@ -11,14 +11,12 @@
 
 // stage kernels of the two builds (stage_exact.cu, stage_fast.cu)
 namespace smaug_exact {
-void launch_stage(int D, bool mixed, const smaug::StageArgs &a, const smaug::Geo &g, const smaug::Phys &p,
-                  cudaStream_t st);
+void launch_stage(int D, const smaug::StageArgs &a, const smaug::Geo &g, const smaug::Phys &p, cudaStream_t st);
 void launch_reduce(int D, const double *w, const double *bg, const smaug::Geo &g, const smaug::Phys &p,
                    smaug::Reduce *r, cudaStream_t st, int const_only = 0);
 }  // namespace smaug_exact
 namespace smaug_fast {
-void launch_stage(int D, bool mixed, const smaug::StageArgs &a, const smaug::Geo &g, const smaug::Phys &p,
-                  cudaStream_t st);
+void launch_stage(int D, const smaug::StageArgs &a, const smaug::Geo &g, const smaug::Phys &p, cudaStream_t st);
 void launch_reduce(int D, const double *w, const double *bg, const smaug::Geo &g, const smaug::Phys &p,
                    smaug::Reduce *r, cudaStream_t st, int const_only = 0);
 }  // namespace smaug_fast

@@ -545,17 +545,17 @@ __device__ __forceinline__ void advance_cell(const StageArgs &a, const Geo &g, c
     neg = (i0 ? g0 : 0u) ^ (i1 ? g1 : 0u) ^ (i2 ? g2 : 0u);
   }
 }
-// The same with the kind at run time (single-step runs).
-template <int D, typename T>
+// The same in FP64 with the kind at run time (tile_body).
+template <int D>
 __device__ __forceinline__ void advance_cell_any(const StageArgs &a, const Geo &g, const Phys &p, const int *c,
-                                                 long long idx, double h, const T *dL, T *red) {
+                                                 long long idx, double h, const double *dL, double *red) {
   const double tdep = p.drv_on ? driver_tdep(p, a.sc, a.tfrac) : 0.0;
   if (a.kind == 3)
-    advance_cell<D, T, 3>(a, g, p, c, idx, h, tdep, dL, red);
+    advance_cell<D, double, 3>(a, g, p, c, idx, h, tdep, dL, red);
   else if (a.kind == 4)
-    advance_cell<D, T, 4>(a, g, p, c, idx, h, tdep, dL, red);
+    advance_cell<D, double, 4>(a, g, p, c, idx, h, tdep, dL, red);
   else
-    advance_cell<D, T, 0>(a, g, p, c, idx, h, tdep, dL, red);
+    advance_cell<D, double, 0>(a, g, p, c, idx, h, tdep, dL, red);
 }
 
 // Divergence-of-B source terms at an inner cell (cudivb, divb.cu:165-336 with
@@ -600,16 +600,16 @@ __device__ __forceinline__ void divb_sources(const CellT<2, T> &C, const Geo &g,
 
 // One RK stage on the tile (bx, by, bz) of one simulation; every thread of
 // the block calls it (it synchronises the block).  sm: tile_smem_elems<D, S>()
-// elements of T.  (Single-step runs, and 3-D runs without the workspace of
-// smaug_pass3.cuh.)
-template <int D, typename T, typename S>
+// doubles.  (Single-step runs, and 3-D runs without the workspace of
+// smaug_pass3.cuh; FP64: mixed runs are RK4 through the batch kernels.)
+template <int D, typename S>
 __device__ __forceinline__ void tile_body(const StageArgs &a, const Geo &g, const Phys &p, int bx, int by, int bz,
-                                          T *sm, T *red) {
+                                          double *sm, double *red) {
+  using T = double;
   using L = Lay<D>;
   constexpr int TX = S::TX, TY = S::TY, TZ = S::TZ, NT = TX * TY * TZ;
   constexpr int NW = L::NW, NB = L::NVAR - NW;
   constexpr int NQ = 2 * D + 1;  // q slots per cell for one dimension
-  constexpr bool MIXED = sizeof(T) == sizeof(float);
 
   const int t = threadIdx.x;
   const int tc[3] = {t % TX, (t / TX) % TY, D == 3 ? t / (TX * TY) : 0};
@@ -620,7 +620,7 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, const Geo &g, cons
   for (int d = 0; d < D; ++d)
     if (c[d] > g.n[d] - 3) active = false;
   const long long idx = active ? gidx<D>(g, c) : 0;
-  const CellT<D, T> C{MIXED ? (const T *)(const void *)a.in32 : (const T *)(const void *)a.in, a.bg, g.N};
+  const CellT<D, T> C{a.in, a.bg, g.N};
   const double dt = a.sc->dt;
   const double h = a.hslot > 0 ? a.sc->hst[a.hslot] : dt / a.hdiv;
   T cm[3] = {0, 0, 0};
@@ -934,19 +934,19 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, const Geo &g, cons
   }
 
   if (numax > red[5] || numax != numax) red[5] = numax;
-  if (active) advance_cell_any<D, T>(a, g, p, c, idx, h, dL, red);
+  if (active) advance_cell_any<D>(a, g, p, c, idx, h, dL, red);
 }
 
 // One launch = one RK stage of one simulation, one block per tile.
-template <int D, typename T>
+template <int D>
 __global__ void __launch_bounds__(256, 2) tile_stage_kernel(StageArgs a, Geo g, Phys p) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  T red[6] = {0, 0, 0, 0, 0, 0};
-  tile_body<D, T, TileShape<D>>(a, g, p, blockIdx.x, blockIdx.y, blockIdx.z, reinterpret_cast<T *>(smraw), red);
+  double red[6] = {0, 0, 0, 0, 0, 0};
+  tile_body<D, TileShape<D>>(a, g, p, blockIdx.x, blockIdx.y, blockIdx.z, reinterpret_cast<double *>(smraw), red);
   block_max_flush<0, 6>(red, &a.sc->red[a.red_out]);
 }
 
-// shared memory elements (of the stencil type) the tile body needs
+// shared memory elements the tile body needs
 template <int D, typename S = TileShape<D>>
 __host__ __device__ constexpr int tile_smem_elems() {
   constexpr int NW = 2 + 2 * D, NQ = 2 * D + 1;

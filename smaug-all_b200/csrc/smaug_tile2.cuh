@@ -167,14 +167,14 @@ __device__ __forceinline__ void prefetch_qbox_rows(const StageArgs &a, const Geo
   }
 }
 
-template <typename T, typename S>
-__device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, const Phys &p, const T *scm, int bx, int by,
-                                           int nbx, int nby, T *sm, T &red) {
+template <typename S>
+__device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, const Phys &p, const double *scm, int bx,
+                                           int by, int nbx, int nby, double *sm, double &red) {
+  using T = double;
   using L = Lay<2>;
   using B = Box2<S>;
   constexpr int TX = S::TX, TY = S::TY, NT = TX * TY;
   constexpr int NW = L::NW;
-  constexpr bool MIXED = sizeof(T) == sizeof(float);
   T *Q = sm + B::OQ, *V0 = sm + B::OV0, *V1 = sm + B::OV1;
 
   const int t = threadIdx.x;
@@ -188,7 +188,7 @@ __device__ __forceinline__ void tile_body2(const StageArgs &a, const Geo &g, con
   int c[3] = {ox + t % TX, oy + (PAIRED ? ((t >> 4) & 1) * (TY / 2) + (t >> 5) : t / TX), 0};
   const bool active = c[0] <= n0 - 3 && c[1] <= n1 - 3;
   const long long idx = active ? c[0] + (long long)c[1] * g.st[1] : 0;
-  const CellT<2, T> C{MIXED ? (const T *)(const void *)a.in32 : (const T *)(const void *)a.in, a.bg, g.N};
+  const CellT<2, T> C{a.in, a.bg, g.N};
   const T cm[2] = {scm[0], scm[1]};  // c_max of the stage input
   if (nbx >= 0) prefetch_qbox_rows<T, TX, TY, NT>(a, g, p, nbx, nby);
 
