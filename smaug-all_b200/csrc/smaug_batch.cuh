@@ -17,7 +17,7 @@ struct BatchInst {
   double *W[4];      // FP64 path: state and the three RK stage buffers; mixed: W[0] only (load/store)
   float *F[5];       // mixed path: w32, c32, two FP32 stage states, FP32 RK sum
   DevScalars *sc;
-  int tiles[3];      // tiles per dimension for the batch's current tile shape
+  int tiles[3];      // 2-D: tiles per dimension for the batch's current tile shape
   int active;        // slot holds a simulation
 };
 

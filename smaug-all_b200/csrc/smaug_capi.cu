@@ -129,8 +129,9 @@ void launch_stage(Run &r, const StageArgs &a) {
   });
 }
 
-// RK stage k (1..4) of the production path: the batch stage kernel, one
-// block per tile of this simulation.
+// RK stage k (1..4) of the production path: the batch kernels over this
+// simulation (2-D: the stage kernel over its tiles; 3-D: the three passes), and
+// the advance pass.
 void launch_rk_stage(Run &r, int k) {
   timed_launch(r, [&] {
     const int v = batch_default_variant(r.D, r.mixed);

@@ -1,18 +1,20 @@
 // smaug_device.cuh -- device side of the fused ideal-MHD stage (sm_100a).
 //
-// One thread advances one interior cell through one Runge-Kutta stage:
+// A Runge-Kutta stage advances the interior cells by
 //   out = base + h * L(in)
 // where L is the SMAUG/SAC single-step operator (fluxes + divergence, the
 // background energy terms, gravity, hyperdiffusive viscosity/resistivity).
 // The reference runs L as ~300 separate kernels that round-trip every
-// intermediate through HBM (dev/smaug/src/iosmaug.cpp:904-1166); here the
-// whole operator is evaluated in registers from the state of the cell's
-// neighbourhood and written once, together with the ghost copies of the
-// cell (the on-device replacement for cuboundary / the MPI halo exchange).
+// intermediate through HBM (dev/smaug/src/iosmaug.cpp:904-1166); here a stage is
+// one to four kernels, the last of which writes each cell together with its ghost
+// copies (the on-device replacement for cuboundary / the MPI halo exchange).
 //
-// Each increment is applied in the order the reference applies it to its
-// output slot, and with the same expression shapes; built without FMA
-// contraction this reproduces the oracle (and so the reference) bit for bit.
+// The functions here form L term by term: each increment in the order the
+// reference applies it to its output slot, and with the same expression shapes;
+// built without FMA contraction (smaug_stage.cuh, one thread per cell, all of L in
+// registers) they reproduce the oracle (and so the reference) bit for bit.  The
+// production kernels (batch_kernels.inc) share the layouts, the boundary rules,
+// the scalars and the driver, and form L by their own arrangement.
 //
 // Field ids follow iotypes.h:213-219; evolved fields live in the state
 // buffers, the static background fields (eb, rhob, bb...) in `bg`.

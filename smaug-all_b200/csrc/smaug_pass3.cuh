@@ -12,8 +12,8 @@
 //   terms    every inner cell: flux divergences, gravity, background energy
 //            terms and hyperdiffusion; the sources go to the advance pass.
 // A slab is a range of planes: it bounds the workspace (kSlabBytes).
-// Blast wave 128^3, mixed (ncu, one stage): derive 47 us, faces 91 us and terms
-// 225 us with the workspace partly from HBM (0.85 KB of traffic per cell), where
+// Blast wave 128^3, mixed (ncu, one stage): derive 38 us, faces 88 us and terms
+// 226 us with the workspace partly from HBM (0.85 KB of traffic per cell), where
 // the tile kernel took 740 us with its epilogue.
 //
 // Workspace of a slab (elements of the stencil type T, vectors so that a

@@ -1,8 +1,10 @@
-// smaug_tile.cuh -- production stage kernel: shared-memory tiles, each
-// per-cell quantity, flux and hyperviscosity computed once per tile.
+// smaug_tile.cuh -- what the production stage kernels share (arithmetic in the
+// stencil type, the advance pass with its ghost images and wave-speed maxima, the
+// divergence-of-B terms), and the FP64 tile kernel that runs a whole stage of one
+// simulation by itself: single-step runs, and 3-D RK4 without a workspace.
 //
 // Same operator as smaug_stage.cuh (the term-by-term restatement used for
-// bit-exact parity), reorganised for throughput:
+// bit-exact parity), reorganised for throughput.  In the tile kernel
 //  * a block owns a TX x TY (x TZ) tile of inner cells, one thread per cell;
 //  * fluxes of every field along `dir` are evaluated once on the tile widened
 //    by 2 along dir and kept in shared memory for the 5-point divergence;
@@ -19,8 +21,7 @@
 // path keeps FP64 where accuracy needs it: the background fields, the total
 // pressure p_T and the internal energy (both recovered by cancellation), the
 // RK base state (an FP32 value plus an FP32 compensation), the RK combination
-// itself and the dt reductions.  With T = double every expression below is
-// the FP64 path's.
+// itself and the dt reductions.
 #pragma once
 #include <type_traits>
 #include "smaug_device.cuh"
