@@ -889,6 +889,7 @@ int smaug_batch_tune(smaug_batch *b, int reps, int *variant_out, double *ms_out,
   BK(cudaEventCreate(&e1));
   int best = b->variant;
   float best_ms = 1e30f;
+  std::vector<std::pair<int, int>> alike;  // a variant, and the one that is timed for it
   for (int v = 0; v < nv; ++v) {
     // a shape that cannot be resident on this device (its shared memory or
     // registers) is not timed: ms -1
@@ -897,16 +898,20 @@ int smaug_batch_tune(smaug_batch *b, int reps, int *variant_out, double *ms_out,
       if (ms_out && v < nms) ms_out[v] = -1.0;
       continue;
     }
-    // the same launches as an earlier variant's: its time, timed once
-    const int first = batch_first_alike(b->D, v);
-    if (first < v) {
-      if (ms_out && v < nms) ms_out[v] = ms_out[first];
+    // the same launches as another variant's are timed once, as that one (in 2-D
+    // that depends on the tiles)
+    int same = b->D == 3 ? batch_alike(3, b->mixed, v, 0, 0) : v;
+    if (same == v) {
+      b->variant = v;
+      int rc = rebuild(b);
+      if (rc != SMAUG_OK) return rc;
+      if (b->nwork == 0) break;
+      if (b->D == 2) same = batch_alike(2, b->mixed, v, b->nwork, b->sms);
+    }
+    if (same != v) {
+      alike.push_back({v, same});
       continue;
     }
-    b->variant = v;
-    int rc = rebuild(b);
-    if (rc != SMAUG_OK) return rc;
-    if (b->nwork == 0) break;
     batch_go_kernel<<<(b->max_inst + 127) / 128, 128, 0, b->stream>>>(b->d_tab, b->max_inst);
     launch_rk_stage(b, 1, b->stream);
     BK(cudaEventRecord(e0, b->stream));
@@ -932,6 +937,8 @@ int smaug_batch_tune(smaug_batch *b, int reps, int *variant_out, double *ms_out,
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  for (const auto &a : alike)
+    if (ms_out && a.first < nms) ms_out[a.first] = ms_out[a.second];
   b->variant = best;
   b->dirty = true;
   if (variant_out) *variant_out = best;

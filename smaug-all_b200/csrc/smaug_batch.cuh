@@ -280,10 +280,21 @@ __host__ __device__ inline void batch_tile_shape(int D, int v, int *t) {
   t[2] = b.t[2];
 }
 
-// The first variant that launches what variant v does.
-__host__ __device__ inline int batch_first_alike(int D, int v) {
-  if (D == 2) return v;
-  const BatchVariant b = batch_variant(3, v);
+// Do the 2-D mixed stage's tiles run one cell per thread (twice the threads of the
+// pairs, one kernel for all occupancy targets)?  16x16 tiles, at most two of them
+// per SM (us per step of a vortex, one cell / pairs: 12 tiles 50.4 / 63.1, 144
+// 54.7 / 64.2, 256 68.2 / 70.5, 400 95.5 / 77.2, 1024 144 / 125).  The batch's list
+// has the tiles of all its simulations.
+__host__ __device__ inline bool batch_single_cells(int tx, int ty, int tiles, int sms) {
+  return tx == 16 && ty == 16 && tiles <= 2 * sms;
+}
+
+// The variant that stands for those that launch what variant v does over `tiles`
+// tiles: in 3-D the first of its shape, in 2-D mixed, where all 16x16 tiles run one
+// cell per thread, the default.
+__host__ __device__ inline int batch_alike(int D, bool mixed, int v, int tiles, int sms) {
+  const BatchVariant b = batch_variant(D, v);
+  if (D == 2) return mixed && batch_single_cells(b.t[0], b.t[1], tiles, sms) ? batch_default_variant(2, true) : v;
   for (int u = 0; u < v; ++u) {
     const BatchVariant a = batch_variant(3, u);
     if (a.t[0] == b.t[0] && a.t[1] == b.t[1] && a.t[2] == b.t[2]) return u;
